@@ -329,7 +329,11 @@ int vdi_mg_destroy(vdi_mg* mg);
 /* tgmg::setup: builds the level hierarchy (also done by create). */
 int vdi_mg_setup(vdi_mg* mg);
 /* tgmg::solve_v_cycle: V-cycles on z (initial guess in, solution out) until
- * ||b-Az||_2 <= rtol*||b||_2; precision is a vdi_mg_precision. */
+ * ||b-Az||_2 <= rtol*||b||_2; precision is a vdi_mg_precision. Where the
+ * finest level is solved exactly in place of V-cycles (MAC and FEM systems of
+ * up to a few thousand points a side), vcycles and max_vcycles count that
+ * solve as the V-cycles it stands for: one per 1.25 (FEM 2.5) decades of
+ * residual. A max_vcycles at or below that count runs V-cycles. */
 typedef struct vdi_mg_result {
     int vcycles;
     double rel_res;

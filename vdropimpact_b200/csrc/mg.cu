@@ -2092,6 +2092,7 @@ __global__ void sub_mean_k(const double* src, double* dst, long N, const double*
 #include "mg_general.cuh"
 #include "mg_cluster.cuh"
 #include "mg_fast.cuh"
+#include "mg_direct.cuh"
 
 class MG {
   public:
@@ -2136,6 +2137,10 @@ class MG {
     FastArrays<double> fc64;
     FastArrays<float> fc32;
     bool allow_fast = true;      // false where its arrays would need an allocation
+    // the exact solve of the finest level (mg_direct.cuh), when the grid has one
+    bool direct = false, dr_blue = false;
+    DirectPlan dr;
+    void* dr_arena = nullptr;
     // the cluster-resident coarse cycle (mg_cluster.cuh) of the FP64 and FP32
     // V-cycles: its top level (-1: not used), CTAs and shared memory per CTA
     struct ClusterPlan {
@@ -2169,6 +2174,9 @@ class MG {
         dlev = -1;
         free_gdirect();
         free_fast();
+        if (dr_arena) cudaFree(dr_arena);
+        dr_arena = nullptr;
+        direct = false;
         if (bproj) cudaFree(bproj);
         if (dmean) cudaFree(dmean);
         bproj = nullptr;
@@ -2474,7 +2482,7 @@ class MG {
             };
             VDI_TRY(gen.setup(m, n, apply, neumann()));
             VDI_CUDA(cudaDeviceSynchronize());
-            return VDI_OK;
+            return setup_direct_solve();
         }
         z64.assign(nlev, nullptr); b64.assign(nlev, nullptr);
         z32.assign(nlev, nullptr); b32.assign(nlev, nullptr);
@@ -2511,8 +2519,60 @@ class MG {
         VDI_CUDA(fem_tile_attr<float>());
         VDI_CUDA((fem_tile_attr<double, float>()));
         VDI_TRY(setup_direct());
+        return setup_direct_solve();
+    }
+
+    /** The exact solve of the finest level (mg_direct.cuh) for the MAC and FEM
+     * systems, on every grid it covers. VDI_MG_DIRECT=0 turns it off, as do the
+     * switches that ask for particular V-cycles (VDI_MG_FAST_COARSE=0,
+     * VDI_MG_GENERAL). */
+    int setup_direct_solve() {
+        auto is = [](const char* name, bool on) {
+            const char* e = getenv(name);
+            return e && (atoi(e) != 0) == on;
+        };
+        if (!allow_fast || !(mac_like() || fem()) || is("VDI_MG_DIRECT", false) || is("VDI_MG_FAST_COARSE", false) ||
+            is("VDI_MG_GENERAL", true))
+            return VDI_OK;
+        DirectPlan p;
+        bool blue;
+        if (!dr_sizes(m, n, fem(), p, blue)) return VDI_OK;
+        DirectModes M;
+        M.off.resize(m);
+        M.di.resize(m);
+        M.d0.resize(m);
+        M.dt.resize(m);
+        const double PI = 3.14159265358979323846;
+        for (int k = 0; k < m; k++) {
+            if (fem()) {
+                // cos(pi k / (m-1)) of the nodes' x neighbours; half of the
+                // diagonal on the top row
+                const double co = std::cos(PI * k / (m - 1));
+                M.off[k] = fop.fey + 2 * fop.fc * co;
+                M.di[k] = M.d0[k] = fop.fm + 2 * fop.fex * co;
+                M.dt[k] = 0.5 * M.di[k];
+            } else {
+                const double sn = std::sin(0.5 * PI * k / m), lam = -4 * c1 * sn * sn;
+                M.off[k] = c2;
+                M.di[k] = lam - 2 * c2;
+                M.d0[k] = lam - (neumann() ? 1 : 3) * c2;
+                M.dt[k] = lam - c2;
+            }
+        }
+        M.pin0 = neumann();
+        if (fem()) p.row0 = 2.0 / fop.fm;
+        VDI_CUDA(fem() ? dr_prepare<FEMc<double>>(p, blue) : dr_prepare<CCc<double>>(p, blue));
+        VDI_TRY(dr_build(p, fem(), blue, M, &dr_arena));
+        dr = p;
+        dr_blue = blue;
+        direct = true;
         return VDI_OK;
     }
+
+    /** Decades of residual that one V-cycle gains (0.09-0.14 per MAC V-cycle,
+     * below 0.01 per FEM one): the exact solve counts as the V-cycles it
+     * stands for, so counts and caps keep their meaning. */
+    double direct_decades() const { return fem() ? 2.5 : 1.25; }
 
     /** Sweeps on the coarsest level: enough for its few points, few enough
      * that the single-CTA cycle stays short. */
@@ -2912,6 +2972,9 @@ class MG {
      * the residual norm of the new iterate and the solve decision. */
     int enqueue_body(cudaStream_t s, const double* b, double* z, int precision, int use_cond,
                      cudaGraphConditionalHandle h) {
+        // what an exact solve leaves is rounding of z, which FP32 corrections
+        // cannot lower: the V-cycles after it are FP64 ones
+        if (direct) return vcycle64(s, b, z, 1, use_cond, h);
         if (precision == VDI_MG_HYBRID) return vcycle_hybrid(s, b, z, 1, use_cond, h);
         if (precision == VDI_MG_MIXED && !general) {
             VDI_TRY(vcycle32(s));
@@ -2926,9 +2989,29 @@ class MG {
         return VDI_OK;
     }
 
+    /** Whether a Gauss-Seidel sweep comes before the first V-cycle: after an
+     * exact MAC solve that falls short, the residual left is rounding at the
+     * grid's scale (the FEM's lies near 1e-14). */
+    bool polishes() const { return direct && !fem(); }
+    /** The sweep with its norm and decision (not counted as a V-cycle); v is
+     * the condition of the V-cycle behind it when recording a loop. */
+    int enqueue_polish(cudaStream_t s, const double* b, double* z, int use_cond, cudaGraphConditionalHandle h,
+                       cudaGraphConditionalHandle v) {
+        const int nb = std::max(1, std::min(nblk(size(0) / 2 + 1), 8 * resident_blocks() / 6));
+        for (int color = 0; color < 2; color++) dr_relax_k<<<nb, 256, 0, s>>>(ccc<double>(0), z, b, ctl, color);
+        dr_polish_check_k<<<sblk0(), 256, 0, s>>>(ccc<double>(0), z, b, rd, ctl, use_cond, h, v);
+        VDI_CUDA(cudaGetLastError());
+        return VDI_OK;
+    }
+
     int enqueue_first_check(cudaStream_t s, const double* b, double* z, int precision, int use_cond,
                             cudaGraphConditionalHandle h) {
         int nb = sblk0();
+        if (direct) {
+            if (fem())
+                return dr_enqueue(s, femc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, nb, use_cond, h);
+            return dr_enqueue(s, ccc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, nb, use_cond, h);
+        }
         if (precision == VDI_MG_MIXED && !general) {
             if (fem()) first_check_k<double><<<nb, 256, 0, s>>>(femc<double>(0), z, b, rd, ctl, use_cond, h, b32[0]);
             else first_check_k<double><<<nb, 256, 0, s>>>(ccc<double>(0), z, b, rd, ctl, use_cond, h, b32[0]);
@@ -3059,7 +3142,8 @@ int mg_solve(MG* mg, cudaStream_t s, const double* b, double* z, double rtol, in
         VDI_CUDA(cudaMemcpyAsync(&h, mg->ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s));
         VDI_CUDA(cudaStreamSynchronize(s));
         if (h.done) break;
-        VDI_TRY(mg->enqueue_body(s, bb, z, precision, 0, 0));
+        if (h.polish) VDI_TRY(mg->enqueue_polish(s, bb, z, 0, 0, 0));
+        else VDI_TRY(mg->enqueue_body(s, bb, z, precision, 0, 0));
     }
     if (mg->neumann()) {
         VDI_TRY(mg->remove_mean(s, z, z));
@@ -3088,41 +3172,68 @@ int mg_solve_device(MG* mg, cudaStream_t s, const double* b, double* z, int prec
     return mg_solve(mg, s, b, z, mg->rtol, mg->max_it, precision, nullptr, nullptr);
 }
 
-int mg_record_graph_solve(MG* mg, cudaStream_t s, const double* b, double* z, int precision) {
+/** Adds a conditional node of the given type behind what the capture on s
+ * holds so far, on a handle of its graph; *body is the graph it runs. */
+static int add_conditional(cudaStream_t s, cudaGraphConditionalNodeType type, cudaGraphConditionalHandle h,
+                           cudaGraph_t* body) {
     cudaStreamCaptureStatus cs;
     cudaGraph_t g;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
-    VDI_TRY(mg->enqueue_begin(s, b, z));
     VDI_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &ndeps));
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = type;
+    cp.conditional.size = 1;
+    cudaGraphNode_t node;
+    VDI_CUDA(cudaGraphAddNode(&node, g, deps, ndeps, &cp));
+    *body = cp.conditional.phGraph_out[0];
+    VDI_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
+    return VDI_OK;
+}
+
+/** Records what f(stream) launches into graph g. */
+template <class F>
+static int record_into(cudaGraph_t g, F f) {
+    cudaStream_t bs;
+    VDI_CUDA(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
+    cudaError_t e = cudaStreamBeginCaptureToGraph(bs, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
+    if (e != cudaSuccess) {
+        cudaStreamDestroy(bs);
+        VDI_CUDA(e);
+    }
+    const int st = f(bs);
+    cudaGraph_t out;
+    e = cudaStreamEndCapture(bs, &out);
+    cudaStreamDestroy(bs);
+    if (st != VDI_OK) return st;
+    VDI_CUDA(e);
+    return VDI_OK;
+}
+
+int mg_record_graph_solve(MG* mg, cudaStream_t s, const double* b, double* z, int precision) {
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t g;
+    VDI_TRY(mg->enqueue_begin(s, b, z));
+    VDI_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, nullptr, nullptr));
     if (cs != cudaStreamCaptureStatusActive) return VDI_ERR_NOT_READY;
     cudaGraphConditionalHandle h;
     VDI_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
     const double* bb = mg->rhs(b);
     VDI_TRY(mg->enqueue_first_check(s, bb, z, precision, 1, h));
-    VDI_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &ndeps));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    VDI_CUDA(cudaGraphAddNode(&node, g, deps, ndeps, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    VDI_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
-    cudaStream_t bs;
-    VDI_CUDA(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
-    cudaError_t e = cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(bs);
-        VDI_CUDA(e);
-    }
-    int st = mg->enqueue_body(bs, bb, z, precision, 1, h);
-    cudaGraph_t bodyOut;
-    e = cudaStreamEndCapture(bs, &bodyOut);
-    cudaStreamDestroy(bs);
-    if (st != VDI_OK) return st;
-    VDI_CUDA(e);
+    cudaGraph_t body;
+    VDI_TRY(add_conditional(s, cudaGraphCondTypeWhile, h, &body));
+    VDI_TRY(record_into(body, [&](cudaStream_t bs) -> int {
+        if (!mg->polishes()) return mg->enqueue_body(bs, bb, z, precision, 1, h);
+        // the sweep after an exact solve, then a V-cycle if that leaves work
+        cudaGraphConditionalHandle v;
+        VDI_CUDA(cudaGraphConditionalHandleCreate(&v, body, 0, 0));
+        VDI_TRY(mg->enqueue_polish(bs, bb, z, 1, h, v));
+        cudaGraph_t vbody;
+        VDI_TRY(add_conditional(bs, cudaGraphCondTypeIf, v, &vbody));
+        return record_into(vbody, [&](cudaStream_t vs) { return mg->enqueue_body(vs, bb, z, precision, 1, h); });
+    }));
     if (mg->neumann()) VDI_TRY(mg->remove_mean(s, z, z));
     return VDI_OK;
 }
@@ -3148,6 +3259,7 @@ int mg_residual(MG* mg, cudaStream_t s, const double* b, const double* z, double
 
 int mg_kernels_per_iteration(const MG* mg, int precision) {
     if (mg->general) return mg->gen.kernels_per_vcycle() + 1;
+    if (mg->direct) precision = VDI_MG_FP64;
     if (precision == VDI_MG_HYBRID) {
         if (mg->nmulti64 < 1 || mg->nmulti32 < 1) precision = VDI_MG_FP64;
         else return 2 * mg->nmulti32 + 1;
@@ -3158,6 +3270,8 @@ int mg_kernels_per_iteration(const MG* mg, int precision) {
     else if (nm == 0) k += 1;                 // separate norm when no tile level exists
     return k;
 }
+
+int mg_kernels_per_start(const MG* mg) { return mg->direct ? 4 : 1; }
 
 double mg_vcycle_bytes(const MG* mg, int fine_word, int coarse_word) {
     // canonical bytes of a V-cycle: per level, each smoothing sweep reads z

@@ -923,6 +923,7 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
     VDI_CUDA(cudaStreamSynchronize(S->s));
     memset(out, 0, sizeof(*out));
     out->steps = S->steps;
+    long direct[4] = {0, 0, 0, 0};
     for (int k = 0; k < 4; k++) {
         if (!S->mg[k]) continue;
         SolveCtl c;
@@ -930,9 +931,12 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
         out->solves[k] = long(c.solves);
         out->vcycles[k] = long(c.vcycles);
         out->last_rel_res[k] = c.last_rel;
+        direct[k] = long(c.direct_cycles);
         if (reset) {
             c.solves = 0;
             c.vcycles = 0;
+            c.direct_solves = 0;
+            c.direct_cycles = 0;
             VDI_CUDA(cudaMemcpy(mg_ctl(S->mg[k]), &c, sizeof(SolveCtl), cudaMemcpyHostToDevice));
         }
     }
@@ -950,9 +954,10 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
     long launches = S->steps * per_step;
     for (int k = 0; k < 4; k++) {
         if (!S->mg[k]) continue;
-        // the guess kernel and the start check
-        launches += out->solves[k] * 2 +
-                    out->vcycles[k] * mg_kernels_per_iteration(S->mg[k], S->prm.mg_precision);
+        // the guess kernel and the solve's start; the V-cycles an exact
+        // solve counts as were not launched
+        launches += out->solves[k] * (1 + mg_kernels_per_start(S->mg[k])) +
+                    (out->vcycles[k] - direct[k]) * mg_kernels_per_iteration(S->mg[k], S->prm.mg_precision);
     }
     out->kernel_launches = launches;
     GasStats gs;

@@ -56,6 +56,12 @@ struct SolveCtl {
     int sticky;         // DevErr bits of every solve since creation
     int* err_out;       // when set, a failing solve also ORs its bits here
     int tma_timeout;    // set when a tile kernel's bulk copy did not arrive in time
+    // exact solves of the finest level: the V-cycles the current solve's one
+    // counts as (0: it does not run), and the totals since the last reset
+    int direct;
+    int polish;         // 1 between an exact solve that fell short and the sweep after it
+    long long direct_solves;
+    long long direct_cycles;
 };
 
 /** Deterministic block-then-grid sum: each block writes one partial, the
@@ -134,6 +140,9 @@ int mg_tile_path(long long* persistent_launches);
 int mg_record_graph_solve(MG* mg, cudaStream_t s, const double* b, double* z, int precision);
 /** Kernel launches of one solve-loop iteration (a V-cycle and its norm). */
 int mg_kernels_per_iteration(const MG* mg, int precision);
+/** Kernel launches that start a solve: the first check, or the exact solve
+ * of the finest level with its checks. */
+int mg_kernels_per_start(const MG* mg);
 /** Times the finest-level PRE (which=0) or POST (which=1) kernel. */
 int mg_profile(MG* mg, cudaStream_t s, int which, int iters, const double* b, double* z, float* ms,
                double* bytes);
