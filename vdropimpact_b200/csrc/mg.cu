@@ -2093,6 +2093,7 @@ __global__ void sub_mean_k(const double* src, double* dst, long N, const double*
 #include "mg_cluster.cuh"
 #include "mg_fast.cuh"
 #include "mg_direct.cuh"
+#include "mg_relax.cuh"
 
 class MG {
   public:
@@ -2141,6 +2142,9 @@ class MG {
     bool direct = false, dr_blue = false;
     DirectPlan dr;
     void* dr_arena = nullptr;
+    // the SOR solver of a weakly coupled viscous system (mg_relax.cuh)
+    RelaxPlan rx;
+    double* rx_tmp = nullptr;   // its scratch iterate where the hierarchy has none
     // the cluster-resident coarse cycle (mg_cluster.cuh) of the FP64 and FP32
     // V-cycles: its top level (-1: not used), CTAs and shared memory per CTA
     struct ClusterPlan {
@@ -2177,6 +2181,9 @@ class MG {
         if (dr_arena) cudaFree(dr_arena);
         dr_arena = nullptr;
         direct = false;
+        if (rx_tmp) cudaFree(rx_tmp);
+        rx_tmp = nullptr;
+        rx = RelaxPlan{};
         if (bproj) cudaFree(bproj);
         if (dmean) cudaFree(dmean);
         bproj = nullptr;
@@ -2482,6 +2489,7 @@ class MG {
             };
             VDI_TRY(gen.setup(m, n, apply, neumann()));
             VDI_CUDA(cudaDeviceSynchronize());
+            VDI_TRY(setup_relax());
             return setup_direct_solve();
         }
         z64.assign(nlev, nullptr); b64.assign(nlev, nullptr);
@@ -2519,7 +2527,36 @@ class MG {
         VDI_CUDA(fem_tile_attr<float>());
         VDI_CUDA((fem_tile_attr<double, float>()));
         VDI_TRY(setup_direct());
+        VDI_TRY(setup_relax());
         return setup_direct_solve();
+    }
+
+    /** The SOR solver for the viscous systems (mg_relax.cuh) while its rate,
+     * omega - 1 a sweep, is below 0.6 (vfx + vfy up to 7.5). At 2048 x 1024 a
+     * solve to 1e-10 takes V-cycles 419 us at vfx = vfy = 0.4, 657 at 1 and 829
+     * at 3, this 187 us at 0.4 and 306 at 2; past the line its passes would
+     * outnumber the V-cycles.
+     * VDI_MG_SOR=0 and VDI_MG_GENERAL turn it off. */
+    int setup_relax() {
+        const char* e = getenv("VDI_MG_SOR");
+        const char* g = getenv("VDI_MG_GENERAL");
+        if ((e && atoi(e) == 0) || (g && atoi(g) != 0)) return VDI_OK;
+        if ((kind != VDI_MG_VISC_U && kind != VDI_MG_VISC_V) || m < 3 || n < 3 || !(c1 >= 0 && c2 >= 0)) return VDI_OK;
+        const double sum = 2 * (c1 + c2), rho = sum / (1 + sum), om = 2 / (1 + std::sqrt(1 - rho * rho));
+        if (!(om - 1 <= 0.6)) return VDI_OK;
+        VDI_CUDA(rx_prepare());
+        // the odd passes write the finest tiled level's scratch iterate
+        if (!general && nmulti64 > 0 && t64[0]) {
+            rx.tmp = t64[0];
+        } else {
+            VDI_CUDA(cudaMalloc(&rx_tmp, size(0) * sizeof(double)));
+            rx.tmp = rx_tmp;
+        }
+        rx.rho2 = rho * rho;
+        rx.om_inf = om;
+        rx.R = rx_rows(m, n);
+        rx.on = true;
+        return VDI_OK;
     }
 
     /** The exact solve of the finest level (mg_direct.cuh) for the MAC and FEM
@@ -2972,6 +3009,7 @@ class MG {
      * the residual norm of the new iterate and the solve decision. */
     int enqueue_body(cudaStream_t s, const double* b, double* z, int precision, int use_cond,
                      cudaGraphConditionalHandle h) {
+        if (rx.on) return enqueue_relax(s, b, z, 2, use_cond, h);
         // what an exact solve leaves is rounding of z, which FP32 corrections
         // cannot lower: the V-cycles after it are FP64 ones
         if (direct) return vcycle64(s, b, z, 1, use_cond, h);
@@ -3004,9 +3042,18 @@ class MG {
         return VDI_OK;
     }
 
+    /** A pair of SOR passes: z to the scratch iterate and back (pass: passes
+     * the solve has behind it; its first pair starts the solve). */
+    int enqueue_relax(cudaStream_t s, const double* b, double* z, int pass, int use_cond,
+                      cudaGraphConditionalHandle h) {
+        VDI_TRY(rx_enqueue(s, ccc<double>(0), rx, pass == 0 ? 0 : 1, pass, z, rx.tmp, b, rd, ctl, use_cond, h));
+        return rx_enqueue(s, ccc<double>(0), rx, 2, pass + 1, rx.tmp, z, b, rd, ctl, use_cond, h);
+    }
+
     int enqueue_first_check(cudaStream_t s, const double* b, double* z, int precision, int use_cond,
                             cudaGraphConditionalHandle h) {
         int nb = sblk0();
+        if (rx.on) return enqueue_relax(s, b, z, 0, use_cond, h);
         if (direct) {
             if (fem())
                 return dr_enqueue(s, femc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, nb, use_cond, h);
@@ -3258,6 +3305,7 @@ int mg_residual(MG* mg, cudaStream_t s, const double* b, const double* z, double
 }
 
 int mg_kernels_per_iteration(const MG* mg, int precision) {
+    if (mg->rx.on) return 1;   // a pass of sweeps counts as one
     if (mg->general) return mg->gen.kernels_per_vcycle() + 1;
     if (mg->direct) precision = VDI_MG_FP64;
     if (precision == VDI_MG_HYBRID) {
@@ -3271,7 +3319,7 @@ int mg_kernels_per_iteration(const MG* mg, int precision) {
     return k;
 }
 
-int mg_kernels_per_start(const MG* mg) { return mg->direct ? 4 : 1; }
+int mg_kernels_per_start(const MG* mg) { return mg->direct ? 4 : (mg->rx.on ? 0 : 1); }
 
 double mg_vcycle_bytes(const MG* mg, int fine_word, int coarse_word) {
     // canonical bytes of a V-cycle: per level, each smoothing sweep reads z
@@ -3559,6 +3607,11 @@ int noalloc_build(const NoallocKey& k, unsigned char* base, MG** out) {
                                                    int(CTA_SMEM_LIMIT));
     if (e == cudaSuccess) e = cc_tile_attr<double>();
     if (e == cudaSuccess) e = fem_tile_attr<double>();
+    // viscous systems relax in the scratch iterate carved above
+    if (e == cudaSuccess && (st = g->setup_relax()) != VDI_OK) {
+        noalloc_drop(g);
+        return st;
+    }
     if (e != cudaSuccess) {
         set_error("vdi_mg_solve_noalloc: %s", cudaGetErrorString(e));
         noalloc_drop(g);
