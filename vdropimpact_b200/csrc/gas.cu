@@ -4,8 +4,9 @@
 // pressure and shear stress — runs inside one launch, so the step needs no
 // host round trip and the launch can overlap the liquid's advection kernels.
 //
-// Tridiagonal systems are solved by cyclic reduction in shared memory when
-// every row is diagonally dominant, and otherwise by Gaussian elimination
+// Tridiagonal systems whose rows are all diagonally dominant are solved by
+// eliminating a few rows per thread and reducing the threads' last rows in
+// parallel (partition_solve), beyond its size by cyclic reduction; others by Gaussian elimination
 // with partial pivoting (the algorithm of LAPACK dgtsv, which the reference
 // calls at tri_solve.cc:28) on one thread.
 //
@@ -20,6 +21,7 @@
 // expression order.
 #include "step_kernels.hh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace vdi {
@@ -95,6 +97,120 @@ __device__ void cyclic_reduction(int n, int Np, double* a, double* b, double* c,
     }
 }
 
+/** A barrier of the block's first count threads (whole warps). */
+__device__ __forceinline__ void part_sync(int count) { asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory"); }
+
+/** Solves the n-row system in a, b, c, d (five contiguous arrays a, b, c, d, x
+ * of length Np >= n, a[0] = c[n-1] = 0), solution in d, by the whole block.
+ * A thread eliminates the first L - 1 of its L consecutive rows in registers;
+ * their last rows form a system of ceil(n / L) rows that is solved by
+ * parallel cyclic reduction, one row a thread, with unit diagonals, by the
+ * warps that hold a row (a barrier of 5 warps takes 20 cycles, of 32 warps
+ * 80).
+ *
+ * Bound: latency. A step is two shared reads, a division and one barrier,
+ * log2(n / L) of them; cyclic reduction in place took twice as many, with
+ * idle threads, a whole block's barrier and two divisions each. The gas
+ * update of about four Newton steps takes 57 us (121 by cyclic reduction) at
+ * m = 2048 and 25 us (53) at m = 256. */
+template <int L>
+__device__ void partition_solve(int n, int Np, double* w) {
+    const int t = threadIdx.x, ns = (n + L - 1) / L, r0 = t * L, nt = (ns + 31) & ~31;
+    if (t >= nt) {
+        __syncthreads();
+        return;
+    }
+    const bool on = t < ns;
+    const int ni = on ? min(L, n - r0) - 1 : 0;
+    double y[L], p[L], q[L], va[L], vb[L], vc[L], vd[L];
+#pragma unroll
+    for (int i = 0; i < L; i++) {
+        const bool in = on && i <= ni;
+        va[i] = in ? w[r0 + i] : 0.;
+        vb[i] = in ? w[Np + r0 + i] : 1.;
+        vc[i] = in ? w[2 * Np + r0 + i] : 0.;
+        vd[i] = in ? w[3 * Np + r0 + i] : 0.;
+    }
+    // interior row i: x_i = y_i - p_i X(previous) - q_i X(own last row)
+    double as = va[0], bs = vb[0], cs = vc[0], ds = vd[0];   // the last row
+    double yl = 0, pl = -1, ql = 0;
+#pragma unroll
+    for (int i = 0; i < L; i++) {
+        y[i] = p[i] = q[i] = 0;
+        if (i < ni) {
+            const double inv = 1. / (i ? fma(-va[i], q[i ? i - 1 : 0], vb[i]) : vb[i]);
+            q[i] = vc[i] * inv;
+            y[i] = (i ? fma(-va[i], y[i ? i - 1 : 0], vd[i]) : vd[i]) * inv;
+            p[i] = (i ? -va[i] * p[i ? i - 1 : 0] : va[i]) * inv;
+            yl = y[i];
+            pl = p[i];
+            ql = q[i];
+        }
+        if (i == ni) {
+            as = va[i];
+            bs = vb[i];
+            cs = vc[i];
+            ds = vd[i];
+        }
+    }
+#pragma unroll
+    for (int i = L - 2; i >= 0; i--)
+        if (i < ni - 1) {
+            const double cp = q[i];
+            y[i] = fma(-cp, y[i + 1], y[i]);
+            p[i] = fma(-cp, p[i + 1], p[i]);
+            q[i] = -cp * q[i + 1];
+        }
+    part_sync(nt);
+    // the next thread's first row, which this last row couples to
+    double* B0 = w;
+    double* B1 = w + 3 * ns;
+    if (on) {
+        B1[t] = ni ? y[0] : 0.;
+        B1[ns + t] = ni ? p[0] : 0.;
+        B1[2 * ns + t] = ni ? q[0] : -1.;
+    }
+    part_sync(nt);
+    const bool nx = t + 1 < ns;
+    const double yn = nx ? B1[t + 1] : 0., pn = nx ? B1[ns + t + 1] : 0., qn = nx ? B1[2 * ns + t + 1] : 0.;
+    const double inv = 1. / fma(-cs, pn, fma(-as, ql, bs));
+    double A = -as * pl * inv, C = -cs * qn * inv, D = fma(-cs, yn, fma(-as, yl, ds)) * inv;
+    if (!on) A = C = D = 0;
+    int k = 0;
+    for (int s = 1; s < ns; s <<= 1, k ^= 1) {
+        // the buffer of two steps ago: every thread has read it by the last barrier
+        double* B = k ? B1 : B0;
+        if (on) {
+            B[t] = A;
+            B[ns + t] = C;
+            B[2 * ns + t] = D;
+        }
+        part_sync(nt);
+        if (on) {
+            const bool l = t >= s, r = t + s < ns;
+            const double Al = l ? B[t - s] : 0., Cl = l ? B[ns + t - s] : 0., Dl = l ? B[2 * ns + t - s] : 0.;
+            const double Ar = r ? B[t + s] : 0., Cr = r ? B[ns + t + s] : 0., Dr = r ? B[2 * ns + t + s] : 0.;
+            const double rb = 1. / fma(-C, Ar, fma(-A, Cl, 1.));
+            D = fma(-C, Dr, fma(-A, Dl, D)) * rb;
+            A = -A * Al * rb;
+            C = -C * Cr * rb;
+        }
+    }
+    part_sync(nt);
+    if (on) w[t] = D;
+    part_sync(nt);
+    const double xp = on && t ? w[t - 1] : 0.;
+    double* d = w + 3 * Np;
+    if (on) {
+#pragma unroll
+        for (int i = 0; i < L; i++) {
+            if (i < ni) d[r0 + i] = fma(-q[i], D, fma(-p[i], xp, y[i]));
+            else if (i == ni) d[r0 + i] = D;
+        }
+    }
+    __syncthreads();
+}
+
 /** Gaussian elimination with partial pivoting on one thread (the algorithm
  * of LAPACK dgtsv). dl = a+1, du = c, du2 scratch of n entries. Returns
  * info (0 ok, k>0: zero pivot at row k). Solution in d. */
@@ -129,7 +245,8 @@ __device__ int gepp_tridiag(int n, double* a, double* b, double* c, double* d, d
     return 0;
 }
 
-/** Solves the system in place (solution in d). Whole block. Returns info
+/** Solves the system in place (solution in d; a, b, c, d and x are contiguous
+ * arrays of length Np). Whole block. Returns info
  * in every thread; *pivoted set when the fallback ran. */
 __device__ int tri_solve_block(int n, int Np, double* a, double* b, double* c, double* d, double* x,
                                double* ws, int* pivoted) {
@@ -143,6 +260,13 @@ __device__ int tri_solve_block(int n, int Np, double* a, double* b, double* c, d
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         if (!(fabs(b[i]) >= fabs(a[i]) + fabs(c[i])) || b[i] == 0) bad = 1;
     bad = __syncthreads_or(bad);
+    if (!bad && n <= 4 * int(blockDim.x)) {
+        // 2 rows a thread while that covers the system
+        if (n <= 2 * int(blockDim.x)) partition_solve<2>(n, Np, a);
+        else partition_solve<4>(n, Np, a);
+        *pivoted = 0;
+        return 0;
+    }
     if (!bad) {
         cyclic_reduction(n, Np, a, b, c, d, x);
         for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = x[i];
@@ -158,7 +282,8 @@ __device__ int tri_solve_block(int n, int Np, double* a, double* b, double* c, d
 
 /** One CTA solves the whole system in shared memory (launch_tri_solve
  * rejects systems that do not fit). */
-__global__ void k_tri_solve(int n, int Np, double* ga, double* gb, double* gc, double* gd, int* out_pivoted) {
+__global__ void __launch_bounds__(GAS_THREADS)
+k_tri_solve(int n, int Np, double* ga, double* gb, double* gc, double* gd, int* out_pivoted) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double ws[33];
     double* a = sm;
@@ -423,6 +548,10 @@ size_t gas_work_doubles(int m) {
 
 static size_t gas_smem_limit() { return 220 * 1024; }
 
+/** Threads for a system of n rows: two rows a thread, at least 256 (barriers
+ * of fewer warps are cheaper, see part_sync), at most GAS_THREADS. */
+static int gas_threads(int n) { return std::min(GAS_THREADS, std::max(256, ((n + 1) / 2 + 31) / 32 * 32)); }
+
 int launch_gas_update(cudaStream_t s, const GasPrm& gp, const Gas& gs, const double* u, const double* v, int pitch,
                       const double* d_vframe, double dt, double* d_time, double* work, int* err, GasStats* stats) {
     size_t bytes = gas_work_doubles(gp.m) * sizeof(double);
@@ -433,7 +562,7 @@ int launch_gas_update(cudaStream_t s, const GasPrm& gp, const Gas& gs, const dou
                                       int(gas_smem_limit())));
         attr_set = true;
     }
-    k_gas_update<<<1, GAS_THREADS, use_smem ? bytes : 0, s>>>(gp, gs, u, v, pitch, d_vframe, dt, d_time, work,
+    k_gas_update<<<1, gas_threads(gp.m + 1), use_smem ? bytes : 0, s>>>(gp, gs, u, v, pitch, d_vframe, dt, d_time, work,
                                                               use_smem, err, stats);
     VDI_CUDA(cudaGetLastError());
     return VDI_OK;
@@ -458,7 +587,7 @@ int launch_tri_solve(cudaStream_t s, int n, double* a, double* b, double* c, dou
                                       int(gas_smem_limit())));
         attr_set = true;
     }
-    k_tri_solve<<<1, GAS_THREADS, bytes, s>>>(n, Np, a, b, c, d, d_pivoted);
+    k_tri_solve<<<1, gas_threads(n), bytes, s>>>(n, Np, a, b, c, d, d_pivoted);
     VDI_CUDA(cudaGetLastError());
     return VDI_OK;
 }
