@@ -566,7 +566,11 @@ class TriSolve:
 
     def solve_lapack(self):
         torch = _torch()
-        dev = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (self.a, self.b, self.c, self.d)]
+        host = [np.ascontiguousarray(x) for x in (self.a, self.b, self.c, self.d)]
+        if all(x.dtype == np.float64 and x.shape == host[0].shape for x in host):
+            dev = torch.from_numpy(np.stack(host)).cuda()   # one copy for the four arrays
+        else:
+            dev = [torch.from_numpy(x).cuda() for x in host]
         piv = C.c_int()
         torch.cuda.synchronize()
         check(lib().vdi_tri_solve(self.m, *[C.c_void_p(t.data_ptr()) for t in dev], None, C.byref(piv)),
