@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -183,6 +184,31 @@ __global__ void __launch_bounds__(256) conv3x3_k(ConvArgs<TIN, TOUT> a) {
     }
 }
 
+/** Eight channels (from c, a multiple of 8) of the convolution input at
+ * (y, x) of the operating grid, as src_at gives them; zero outside. */
+__device__ __forceinline__ uint4 src8_at(const bf16* src, int mode, int H, int W, int C, int b, int y, int x, int c) {
+    if (y < 0 || y >= H || x < 0 || x >= W) return make_uint4(0, 0, 0, 0);
+    if (mode == SRC_DIRECT) return *reinterpret_cast<const uint4*>(src + ((size_t(b) * H + y) * W + x) * C + c);
+    if (mode == SRC_UP2)
+        return *reinterpret_cast<const uint4*>(src + ((size_t(b) * (H >> 1) + (y >> 1)) * (W >> 1) + (x >> 1)) * C + c);
+    float s[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) s[k] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const uint4 v = *reinterpret_cast<const uint4*>(
+            src + ((size_t(b) * H * 2 + 2 * y + (d >> 1)) * W * 2 + 2 * x + (d & 1)) * C + c);
+        const bf16* e = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+        for (int k = 0; k < 8; k++) s[k] += __bfloat162float(e[k]);
+    }
+    uint4 r;
+    bf16* e = reinterpret_cast<bf16*>(&r);
+#pragma unroll
+    for (int k = 0; k < 8; k++) e[k] = __float2bfloat16(0.25f * s[k]);
+    return r;
+}
+
 // ------------------------------------------- Blackwell tensor-core path
 // The same convolution on the fifth-generation tensor cores (the default
 // path; VDI_UNET_TC=0 keeps the mma.sync kernel above): tcgen05.mma with
@@ -195,14 +221,16 @@ __global__ void __launch_bounds__(256) conv3x3_k(ConvArgs<TIN, TOUT> a) {
 // [tap][cout][cin], are K-major B operands. A CTA stages the weights once and
 // then walks a contiguous run of segments, consecutive rows of one segment
 // where it can, keeping the input rows in a ring of four: a new segment
-// stages one row, while the tensor cores work on the previous one. Each
-// segment is 9 * CIN/16 MMAs (K = 16 each) into one accumulator, read back
+// stages one row (BF16 sources read as they are by asynchronous 16-byte
+// copies), while the tensor cores work on the previous one. Several CTAs
+// share an SM (tc_blocks), so one's staging and epilogue overlap another's
+// MMAs. Each segment is 9 * CIN/16 MMAs (K = 16 each) into one accumulator, read back
 // with tcgen05.ld for the bias, skip-add, ReLU epilogue.
 namespace tc {
 
 constexpr int TC_M = 128;            // output pixels per segment (MMA M)
 constexpr int TC_PX = TC_M + 2;      // staged pixels per input row (one halo pixel each side)
-constexpr int TC_THREADS = 128;
+constexpr int TC_THREADS = 256;     // all stage rows, the first four warps read the accumulator
 constexpr int TC_RING = 4;           // staged input rows: three in use, the next being loaded
 
 __device__ int g_timeout;            // set when a bounded wait gave up
@@ -288,6 +316,14 @@ constexpr size_t tc_smem() {
     return size_t(9) * (CIN / 8) * COUT * 16 + size_t(TC_RING) * (CIN / 8) * TC_PX * 16 + TC_PAD;
 }
 
+/** CTAs of conv3x3_tc that an SM holds: by shared memory, at most four (of 32
+ * or 64 tensor-memory columns each). The occupancy query answers one. */
+template <int CIN, int COUT>
+constexpr int tc_blocks() {
+    const int by_smem = int(size_t(227 * 1024) / (tc_smem<CIN, COUT>() + 2048));
+    return by_smem < 1 ? 1 : (by_smem > 4 ? 4 : by_smem);
+}
+
 template <int CIN, int COUT, typename TIN, typename TOUT>
 __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) {
     constexpr int KC = CIN / 8;                              // 16-byte channel chunks
@@ -332,44 +368,52 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
     // (yy + 1) % TC_RING, as 16-byte channel chunks
     auto stage = [&](int b, int yy, int x0) {
         unsigned char* dst = rows + uint32_t((yy + 1 + TC_RING) % TC_RING) * ROWB;
-        for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
-            const int px = q % TC_PX, kc = q / TC_PX;
-            const int xx = x0 + px - 1;
-            uint4 v;
-            const bool in = yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-            const size_t k8 = ((size_t(b) * a.H + yy) * a.W + xx) * CIN + kc * 8;
-            if (std::is_same<TIN, bf16>::value && a.mode == SRC_DIRECT && !a.mask) {
-                v = in ? *reinterpret_cast<const uint4*>(a.src + k8) : make_uint4(0, 0, 0, 0);
-            } else if (std::is_same<TIN, float>::value && a.mode == SRC_DIRECT) {
-                // FP32 source (the input gradient's dY), 8 channels in two
-                // 16-byte loads, the ReLU mask as one 16-byte load
-                __align__(16) bf16 e[8];
-                if (in) {
-                    const float4 lo = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.src) + k8);
-                    const float4 hi = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.src) + k8 + 4);
+        const bool rin = yy >= 0 && yy < a.H;
+        if constexpr (std::is_same<TIN, bf16>::value) {
+            if (a.mode == SRC_DIRECT) {
+                const bf16* row = a.src + (size_t(b) * a.H + (rin ? yy : 0)) * a.W * CIN;
+                for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
+                    const int kc = q % KC, px = q / KC, xx = x0 + px - 1;
+                    const bool in = rin && xx >= 0 && xx < a.W;
+                    const int bytes = in ? 16 : 0;   // 0: zero-filled
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                     smem_u32(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16)),
+                                 "l"(row + (in ? size_t(xx) * CIN + kc * 8 : 0)), "r"(bytes)
+                                 : "memory");
+                }
+            } else {
+#pragma unroll 2
+                for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
+                    const int kc = q % KC, px = q / KC;
+                    *reinterpret_cast<uint4*>(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16) =
+                        src8_at(a.src, a.mode, a.H, a.W, CIN, b, yy, x0 + px - 1, kc * 8);
+                }
+            }
+        } else {
+            // FP32 source (the input gradient's dY, read directly), 8 channels
+            // in two 16-byte loads, the ReLU mask as one 16-byte load
+#pragma unroll 2
+            for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
+                const int kc = q % KC, px = q / KC, xx = x0 + px - 1;
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if (rin && xx >= 0 && xx < a.W) {
+                    const size_t k8 = ((size_t(b) * a.H + yy) * a.W + xx) * CIN + kc * 8;
+                    const float4 lo = *reinterpret_cast<const float4*>(a.src + k8);
+                    const float4 hi = *reinterpret_cast<const float4*>(a.src + k8 + 4);
                     float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
                     if (a.mask) {
-                        __align__(16) bf16 mk[8];
-                        *reinterpret_cast<uint4*>(mk) = *reinterpret_cast<const uint4*>(a.mask + k8);
+                        const uint4 mv = *reinterpret_cast<const uint4*>(a.mask + k8);
+                        const bf16* mk = reinterpret_cast<const bf16*>(&mv);
 #pragma unroll
                         for (int c = 0; c < 8; c++)
                             if (!(__bfloat162float(mk[c]) > 0.f)) f[c] = 0.f;
                     }
+                    bf16* e = reinterpret_cast<bf16*>(&v);
 #pragma unroll
                     for (int c = 0; c < 8; c++) e[c] = __float2bfloat16(f[c]);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; c++) e[c] = __float2bfloat16(0.f);
                 }
-                v = *reinterpret_cast<const uint4*>(e);
-            } else {
-                __align__(16) bf16 e[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++)
-                    e[c] = __float2bfloat16(src_at(a.src, a.mask, a.mode, a.H, a.W, CIN, b, yy, xx, kc * 8 + c));
-                v = *reinterpret_cast<const uint4*>(e);
+                *reinterpret_cast<uint4*>(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16) = v;
             }
-            *reinterpret_cast<uint4*>(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16) = v;
         }
     };
     uint32_t phase = 0;
@@ -384,6 +428,7 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
             stage(b, y, x0);
             stage(b, y + 1, x0);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         fence_async_smem();   // the staged rows (and weights) become visible to the tensor cores
         fence_before();
         __syncthreads();
@@ -414,7 +459,7 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
         phase ^= 1;
         ok = __syncthreads_and(ok);
         fence_after();
-        if (ok) {
+        if (ok && warp < 4) {
             const int x = x0 + warp * 32 + lane;
             const uint32_t ta = tmem + (uint32_t(warp * 32) << 16);
 #pragma unroll
@@ -424,13 +469,38 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (x < a.W) {
                     const size_t k = ((size_t(b) * a.H + y) * a.W + x) * COUT + c0;
+                    if (a.bias) {
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        float w = v[c];
-                        if (a.bias) w += a.bias[c0 + c];
-                        if (a.resid) w += __bfloat162float(a.resid[k + c]);
-                        if (a.relu) w = fmaxf(w, 0.f);
-                        a.out[k + c] = from_f<TOUT>(w);
+                        for (int c = 0; c < 16; c++) v[c] += __ldg(a.bias + c0 + c);
+                    }
+                    if (a.resid) {
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const uint4 rv = *reinterpret_cast<const uint4*>(a.resid + k + 8 * h);
+                            const bf16* r = reinterpret_cast<const bf16*>(&rv);
+#pragma unroll
+                            for (int c = 0; c < 8; c++) v[8 * h + c] += __bfloat162float(r[c]);
+                        }
+                    }
+                    if (a.relu) {
+#pragma unroll
+                        for (int c = 0; c < 16; c++) v[c] = fmaxf(v[c], 0.f);
+                    }
+                    // 16 channels of a pixel as 16-byte stores
+                    if constexpr (std::is_same<TOUT, float>::value) {
+#pragma unroll
+                        for (int h = 0; h < 4; h++)
+                            *reinterpret_cast<float4*>(a.out + k + 4 * h) =
+                                make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            uint4 o;
+                            bf16* e = reinterpret_cast<bf16*>(&o);
+#pragma unroll
+                            for (int c = 0; c < 8; c++) e[c] = __float2bfloat16(v[8 * h + c]);
+                            *reinterpret_cast<uint4*>(a.out + k + 8 * h) = o;
+                        }
                     }
                 }
             }
@@ -439,6 +509,7 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
         __syncthreads();   // accumulator read and staged rows consumed before the next segment
         fence_after();
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (!ok) {
         // a wait gave up: note it, and give any MMA still in flight a bounded
         // time to finish before the tensor memory is released
@@ -459,87 +530,159 @@ constexpr size_t conv_smem() {
     return (size_t(TPY + 2) * (TPX + 2) * (CIN + 8) + size_t(9) * COUT * (CIN + 8)) * sizeof(bf16);
 }
 
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+
+/** Shape of the weight-gradient GEMM of one layer: M = output channels, N =
+ * input channels for each of the 9 taps, K = pixels. A warp takes 16 x 8 PN
+ * of (M, N) for all taps in registers; NG warps cover (M, N), and the other
+ * factor KS of the block's eight splits the pixels. */
+template <int CIN, int COUT>
+struct WGrad {
+    static constexpr int TW = 32, TH = 8, NPX = TW * TH, XW = TW + 2, XPX = XW * (TH + 2);
+    static constexpr int GS = COUT + 8, XS = CIN + 8;   // pixel strides: 16 bytes off a multiple of 128
+    static constexpr int MT = COUT / 16, NT = CIN / 8, PN = NT < 4 ? NT : 4, NG = MT * (NT / PN), KS = 8 / NG;
+    static constexpr size_t TILE = (size_t(NPX) * GS + size_t(XPX) * XS) * sizeof(bf16);
+    static constexpr size_t RED = KS > 1 ? size_t(9) * COUT * CIN * sizeof(float) : 0;
+    static constexpr size_t SMEM = TILE > RED ? TILE : RED;
+    static constexpr int MINB = PN == 4 ? 1 : 2;
+};
+
 /** Weight gradient dW[tap][co][ci] += sum_p G[p][co] X_tap[p][ci] and bias
  * gradient, with G = dY masked by the layer's ReLU (mask = layer output) and
- * X the (resampled) layer input. grid.x CTAs stride over pixel tiles,
- * grid.y = 9 taps. Each CTA accumulates in registers and adds once. */
+ * X the (resampled) layer input, on mma.sync m16n8k16 with both operands
+ * read by transposing ldmatrix from pixel-major tiles. A block walks tiles of
+ * 8 rows of 32 pixels: a tile (and X's halo) is staged once for all nine taps,
+ * whose accumulators stay in registers until the end, when the pixel-splitting
+ * warps add up in shared memory and the block adds its sums to dW.
+ *
+ * Bound: reading dY (FP32), the mask and X once, 8 (bytes) COUT + 2 CIN a
+ * pixel. At 8 x 256 x 512 pixels 16 -> 16 takes 76 us (134 MB, 1.8 TB/s), 32 ->
+ * 32 at half the side 71 us; with one tap a block (everything read nine
+ * times, element by element) they took 975 and 468 us. */
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) conv_wgrad_k(const bf16* src, int mode, const float* dy, const bf16* ymask,
-                                                    float* dw, float* db, int B, int H, int W) {
-    constexpr int GS = COUT + 8, XS = CIN + 8;
-    constexpr int NPX = TPX * TPY;
-    __shared__ __align__(16) bf16 gsm[NPX * GS];
-    __shared__ __align__(16) bf16 xsm[NPX * XS];
-    const int tap = blockIdx.y, ky = tap / 3 - 1, kx = tap % 3 - 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, tq = lane & 3;
-    constexpr int MT = COUT / 16, NT = CIN / 8, TILES = MT * NT;
-    constexpr int PER = (TILES + 7) / 8;     // (m,n) tiles per warp
-    float acc[PER][4];
+__global__ void __launch_bounds__(256, WGrad<CIN, COUT>::MINB)
+conv_wgrad_k(const bf16* __restrict__ src, int mode, const float* __restrict__ dy, const bf16* __restrict__ ymask,
+             float* dw, float* db, int B, int H, int W) {
+    using S = WGrad<CIN, COUT>;
+    constexpr int GC = COUT / 8, XC = CIN / 8, TW = S::TW, TH = S::TH;
+    extern __shared__ __align__(16) unsigned char smem[];
+    bf16* gsm = reinterpret_cast<bf16*>(smem);        // [NPX][GS]
+    bf16* xsm = gsm + S::NPX * S::GS;                 // [XPX][XS]
+    __shared__ float bsm[COUT];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gi = warp % S::NG, ki = warp / S::NG;
+    const int m0 = (gi % S::MT) * 16, n0 = (gi / S::MT) * (8 * S::PN);
+    if (tid < COUT) bsm[tid] = 0.f;
+    float acc[9][S::PN][4];
 #pragma unroll
-    for (int q = 0; q < PER; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
-    float bacc = 0.f;
-    const int tilesx = (W + TPX - 1) / TPX, tilesy = (H + TPY - 1) / TPY, ntiles = tilesx * tilesy * B;
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int j = 0; j < S::PN; j++) acc[t][j][0] = acc[t][j][1] = acc[t][j][2] = acc[t][j][3] = 0.f;
+    float bacc[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) bacc[k] = 0.f;
+    static_assert(256 % GC == 0 && 8 % S::NG == 0, "a thread keeps its channels");
+    const int gc = tid % GC, xc = tid % XC;
+    // ldmatrix row addresses of this lane (matrix lane / 8, row lane % 8):
+    // A's matrices run over output channels first, B's over pixels first
+    const int mi = lane >> 3, lr = lane & 7;
+    const int ga = ((mi >> 1) * 8 + lr) * S::GS + m0 + (mi & 1) * 8;
+    const int xa = ((mi & 1) * 8 + lr) * S::XS + n0 + (mi >> 1) * 8;
+    const int tilesx = (W + TW - 1) / TW, tilesy = (H + TH - 1) / TH, ntiles = tilesx * tilesy * B;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int b = tile / (tilesx * tilesy), r = tile % (tilesx * tilesy);
-        const int x0 = (r % tilesx) * TPX, y0 = (r / tilesx) * TPY;
+        const int b = tile / (tilesx * tilesy), r = tile - b * tilesx * tilesy;
+        const int x0 = (r % tilesx) * TW, y0 = (r / tilesx) * TH;
         __syncthreads();
-        for (int t = threadIdx.x; t < NPX * COUT; t += blockDim.x) {
-            int co = t % COUT, p = t / COUT;
-            int x = x0 + p % TPX, y = y0 + p / TPX;
-            float v = 0.f;
+#pragma unroll 4
+        for (int p = tid / GC; p < S::NPX; p += 256 / GC) {
+            const int x = x0 + p % TW, y = y0 + p / TW;
+            uint4 v = make_uint4(0, 0, 0, 0);
             if (x < W && y < H) {
-                size_t k = ((size_t(b) * H + y) * W + x) * COUT + co;
-                v = dy[k];
-                if (ymask && !(__bfloat162float(ymask[k]) > 0.f)) v = 0.f;
+                const size_t k = ((size_t(b) * H + y) * W + x) * COUT + gc * 8;
+                const float4 lo = *reinterpret_cast<const float4*>(dy + k), hi = *reinterpret_cast<const float4*>(dy + k + 4);
+                float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                if (ymask) {
+                    const uint4 mv = *reinterpret_cast<const uint4*>(ymask + k);
+                    const bf16* mk = reinterpret_cast<const bf16*>(&mv);
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        if (!(__bfloat162float(mk[c]) > 0.f)) f[c] = 0.f;
+                }
+                bf16* e = reinterpret_cast<bf16*>(&v);
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    e[c] = __float2bfloat16(f[c]);
+                    bacc[c] += __bfloat162float(e[c]);
+                }
             }
-            gsm[p * GS + co] = __float2bfloat16(v);
+            *reinterpret_cast<uint4*>(gsm + p * S::GS + gc * 8) = v;
         }
-        for (int t = threadIdx.x; t < NPX * CIN; t += blockDim.x) {
-            int ci = t % CIN, p = t / CIN;
-            int x = x0 + p % TPX, y = y0 + p / TPX;
-            float v = (x < W && y < H) ? src_at<bf16>(src, nullptr, mode, H, W, CIN, b, y + ky, x + kx, ci) : 0.f;
-            xsm[p * XS + ci] = __float2bfloat16(v);
-        }
+#pragma unroll 4
+        for (int p = tid / XC; p < S::XPX; p += 256 / XC)
+            *reinterpret_cast<uint4*>(xsm + p * S::XS + xc * 8) =
+                src8_at(src, mode, H, W, CIN, b, y0 + p / S::XW - 1, x0 + p % S::XW - 1, xc * 8);
         __syncthreads();
-        if (tap == 4 && threadIdx.x < COUT) {
-            for (int p = 0; p < NPX; p++) bacc += __bfloat162float(gsm[p * GS + threadIdx.x]);
-        }
+#pragma unroll 1
+        for (int ks = ki; ks < S::NPX / 16; ks += S::KS) {
+            const int row = ks >> 1, cx = (ks & 1) * 16;
+            uint32_t av[4];
+            ldsm_x4_t(av, gsm + (row * TW + cx) * S::GS + ga);
 #pragma unroll
-        for (int q = 0; q < PER; q++) {
-            const int tt = warp + 8 * q;
-            if (tt >= TILES) break;
-            const int mt = tt / NT, nt = tt % NT;
+            for (int t = 0; t < 9; t++) {
+                const bf16* xb = xsm + ((row + t / 3) * S::XW + cx + t % 3) * S::XS + xa;
 #pragma unroll
-            for (int kc = 0; kc < NPX / 16; kc++) {
-                // A = G^T: rows co (mt*16 + ...), cols pixels (kc*16 + ...)
-                const int p0 = kc * 16 + 2 * tq;
-                const int r0 = mt * 16 + g;
-                uint32_t a0 = pack2(gsm[p0 * GS + r0], gsm[(p0 + 1) * GS + r0]);
-                uint32_t a1 = pack2(gsm[p0 * GS + r0 + 8], gsm[(p0 + 1) * GS + r0 + 8]);
-                uint32_t a2 = pack2(gsm[(p0 + 8) * GS + r0], gsm[(p0 + 9) * GS + r0]);
-                uint32_t a3 = pack2(gsm[(p0 + 8) * GS + r0 + 8], gsm[(p0 + 9) * GS + r0 + 8]);
-                // B = X: rows pixels, cols ci (nt*8 + g)
-                const int c0 = nt * 8 + g;
-                uint32_t b0 = pack2(xsm[p0 * XS + c0], xsm[(p0 + 1) * XS + c0]);
-                uint32_t b1 = pack2(xsm[(p0 + 8) * XS + c0], xsm[(p0 + 9) * XS + c0]);
-                mma_bf16(acc[q], a0, a1, a2, a3, b0, b1);
+                for (int j = 0; j < S::PN; j += 2) {
+                    uint32_t bv[4];
+                    ldsm_x4_t(bv, xb + j * 8);
+                    mma_bf16(acc[t][j], av[0], av[1], av[2], av[3], bv[0], bv[1]);
+                    mma_bf16(acc[t][j + 1], av[0], av[1], av[2], av[3], bv[2], bv[3]);
+                }
             }
         }
     }
+    __syncthreads();
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-        const int tt = warp + 8 * q;
-        if (tt >= TILES) break;
-        const int mt = tt / NT, nt = tt % NT;
-        const int co = mt * 16 + g, ci = nt * 8 + 2 * tq;
-        float* d = dw + (size_t(tap) * COUT) * CIN;
-        atomicAdd(d + co * CIN + ci, acc[q][0]);
-        atomicAdd(d + co * CIN + ci + 1, acc[q][1]);
-        atomicAdd(d + (co + 8) * CIN + ci, acc[q][2]);
-        atomicAdd(d + (co + 8) * CIN + ci + 1, acc[q][3]);
+    for (int k = 0; k < 8; k++) atomicAdd(&bsm[gc * 8 + k], bacc[k]);
+    const int g = lane >> 2, tq = lane & 3;
+    if constexpr (S::KS == 1) {
+#pragma unroll
+        for (int t = 0; t < 9; t++)
+#pragma unroll
+            for (int j = 0; j < S::PN; j++) {
+                float* d = dw + (size_t(t) * COUT + m0 + g) * CIN + n0 + j * 8 + 2 * tq;
+                atomicAdd(d, acc[t][j][0]);
+                atomicAdd(d + 1, acc[t][j][1]);
+                atomicAdd(d + 8 * CIN, acc[t][j][2]);
+                atomicAdd(d + 8 * CIN + 1, acc[t][j][3]);
+            }
+        __syncthreads();
+    } else {
+        float* red = reinterpret_cast<float*>(smem);   // [9][COUT][CIN]
+        for (int q = 0; q < S::KS; q++) {
+            if (ki == q) {
+#pragma unroll
+                for (int t = 0; t < 9; t++)
+#pragma unroll
+                    for (int j = 0; j < S::PN; j++) {
+                        float* d = red + (t * COUT + m0 + g) * CIN + n0 + j * 8 + 2 * tq;
+                        float* e = d + 8 * CIN;
+                        d[0] = (q ? d[0] : 0.f) + acc[t][j][0];
+                        d[1] = (q ? d[1] : 0.f) + acc[t][j][1];
+                        e[0] = (q ? e[0] : 0.f) + acc[t][j][2];
+                        e[1] = (q ? e[1] : 0.f) + acc[t][j][3];
+                    }
+            }
+            __syncthreads();
+        }
+        for (int k = tid; k < 9 * COUT * CIN; k += 256) atomicAdd(dw + k, red[k]);
     }
-    if (tap == 4 && threadIdx.x < COUT) atomicAdd(db + threadIdx.x, bacc);
+    if (tid < COUT) atomicAdd(db + tid, bsm[tid]);
 }
 
 /** Flipped, transposed weights for the input gradient:
@@ -686,14 +829,11 @@ static cudaError_t conv_launch(cudaStream_t s, const ConvArgs<TIN, TOUT>& a) {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  int(tc::tc_smem<CIN, COUT>()));
             if (e != cudaSuccess) return e;
-            int dev = 0, sms = 0, per_sm = 0;
+            int dev = 0, sms = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
-                (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-                (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc::conv3x3_tc<CIN, COUT, TIN, TOUT>,
-                                                                   tc::TC_THREADS, tc::tc_smem<CIN, COUT>())) !=
-                    cudaSuccess)
+                (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
                 return e;
-            resident = sms * (per_sm > 0 ? per_sm : 1);
+            resident = sms * tc::tc_blocks<CIN, COUT>();
         }
         const long tasks = long(a.B) * a.H * ((a.W + tc::TC_M - 1) / tc::TC_M);
         const int grid = int(tasks < resident ? tasks : resident);
@@ -722,14 +862,23 @@ static cudaError_t conv_dispatch(cudaStream_t s, int cin, int cout, const ConvAr
     return cudaErrorInvalidValue;
 }
 
+template <int CIN, int COUT>
+static cudaError_t wgrad_launch(cudaStream_t s, const Layer& l, const bf16* src, const float* dy, const bf16* ymask,
+                                int B) {
+    using S = WGrad<CIN, COUT>;
+    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_k<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(S::SMEM));
+    if (e != cudaSuccess) return e;
+    const int tiles = ((l.W + S::TW - 1) / S::TW) * ((l.H + S::TH - 1) / S::TH) * B;
+    conv_wgrad_k<CIN, COUT><<<std::min(tiles, 148 * S::MINB), 256, S::SMEM, s>>>(src, l.mode, dy, ymask, l.g, l.gb, B,
+                                                                                 l.H, l.W);
+    return cudaGetLastError();
+}
+
 static cudaError_t wgrad_dispatch(cudaStream_t s, const Layer& l, const bf16* src, const float* dy, const bf16* ymask,
                                   int B) {
-    dim3 grid(148, 9);
-#define VDI_WG(CI, CO)                                                                                     \
-    if (l.cin == CI && l.cout == CO) {                                                                     \
-        conv_wgrad_k<CI, CO><<<grid, 256, 0, s>>>(src, l.mode, dy, ymask, l.g, l.gb, B, l.H, l.W);        \
-        return cudaGetLastError();                                                                         \
-    }
+#define VDI_WG(CI, CO) \
+    if (l.cin == CI && l.cout == CO) return wgrad_launch<CI, CO>(s, l, src, dy, ymask, B);
     VDI_WG(16, 16) VDI_WG(16, 32) VDI_WG(32, 32) VDI_WG(32, 64) VDI_WG(64, 64) VDI_WG(64, 32) VDI_WG(32, 16)
 #undef VDI_WG
     return cudaErrorInvalidValue;
