@@ -685,66 +685,88 @@ conv_wgrad_k(const bf16* __restrict__ src, int mode, const float* __restrict__ d
     if (tid < COUT) atomicAdd(db + tid, bsm[tid]);
 }
 
-/** Flipped, transposed weights for the input gradient:
- * wt[8-tap][ci][co] = w[tap][co][ci]. */
-__global__ void flip_transpose_k(const bf16* w, bf16* wt, int cin, int cout) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
+/** Flipped, transposed weights for the input gradient of every layer
+ * (blockIdx.y): wt[8-tap][ci][co] = w[tap][co][ci]. */
+struct FlipArgs {
+    const bf16* w[14];
+    bf16* wt[14];
+    int cin[14], cout[14];
+};
+__global__ void flip_transpose_k(FlipArgs a) {
+    const int l = blockIdx.y, cin = a.cin[l], cout = a.cout[l];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 9 * cin * cout) return;
-    int ci = t % cin, r = t / cin, co = r % cout, tap = r / cout;
-    wt[(size_t(8 - tap) * cin + ci) * cout + co] = w[t];
+    const int ci = t % cin, r = t / cin, co = r % cout, tap = r / cout;
+    a.wt[l][(size_t(8 - tap) * cin + ci) * cout + co] = a.w[l][t];
 }
 
-/** dsrc += adjoint of the source resampling applied to dx (operating grid
- * H x W, C channels). */
-__global__ void resample_adjoint_add_k(const float* dx, float* dsrc, int mode, int B, int H, int W, int C) {
-    if (mode == SRC_DIRECT) {
-        size_t n = size_t(B) * H * W * C;
-        for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x)
-            dsrc[k] += dx[k];
-        return;
-    }
-    if (mode == SRC_UP2) {
-        int Hs = H >> 1, Ws = W >> 1;
-        size_t n = size_t(B) * Hs * Ws * C;
-        for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
-            int c = k % C;
-            size_t p = k / C;
-            int xs = p % Ws, ys = (p / Ws) % Hs, b = p / (size_t(Ws) * Hs);
-            float s = 0.f;
-            for (int dy = 0; dy < 2; dy++)
-                for (int dxx = 0; dxx < 2; dxx++) s += dx[((size_t(b) * H + 2 * ys + dy) * W + 2 * xs + dxx) * C + c];
-            dsrc[k] += s;
-        }
-        return;
-    }
-    int Hs = 2 * H, Ws = 2 * W;
-    size_t n = size_t(B) * Hs * Ws * C;
+/** dsrc = the adjoint of nearest upsampling by two applied to dx (operating
+ * grid H x W, C channels): the sum over each source pixel's 2 x 2 block, four
+ * channels a thread. */
+__global__ void upsample_adjoint_k(const float* __restrict__ dx, float* __restrict__ dsrc, int B, int H, int W, int C) {
+    const int Hs = H >> 1, Ws = W >> 1, C4 = C >> 2;
+    const size_t n = size_t(B) * Hs * Ws * C4;
     for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
-        int c = k % C;
-        size_t p = k / C;
-        int xs = p % Ws, ys = (p / Ws) % Hs, b = p / (size_t(Ws) * Hs);
-        dsrc[k] += 0.25f * dx[((size_t(b) * H + ys / 2) * W + xs / 2) * C + c];
+        const int c = int(k % C4);
+        const size_t p = k / C4;
+        const int xs = int(p % Ws), ys = int((p / Ws) % Hs), b = int(p / (size_t(Ws) * Hs));
+        const float4* q = reinterpret_cast<const float4*>(dx + ((size_t(b) * H + 2 * ys) * W + 2 * xs) * C) + c;
+        const float4 v00 = q[0], v01 = q[C4], v10 = q[size_t(W) * C4], v11 = q[size_t(W) * C4 + C4];
+        float4 s;
+        s.x = ((v00.x + v01.x) + v10.x) + v11.x;
+        s.y = ((v00.y + v01.y) + v10.y) + v11.y;
+        s.z = ((v00.z + v01.z) + v10.z) + v11.z;
+        s.w = ((v00.w + v01.w) + v10.w) + v11.w;
+        reinterpret_cast<float4*>(dsrc)[k] = s;
     }
 }
 
-__global__ void add_f32_k(float* a, const float* b, size_t n) {
-    for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x)
-        a[k] += b[k];
+/** dsrc += the adjoint of the 2 x 2 mean applied to dx (operating grid H x W,
+ * C channels): a quarter of each value for its four source pixels, four
+ * channels a thread. */
+__global__ void pool_adjoint_add_k(const float* __restrict__ dx, float* __restrict__ dsrc, int B, int H, int W, int C) {
+    const int Ws = 2 * W, C4 = C >> 2;
+    const size_t n = size_t(B) * 2 * H * Ws * C4;
+    for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
+        const int c = int(k % C4);
+        const size_t p = k / C4;
+        const int xs = int(p % Ws), ys = int((p / Ws) % (2 * H)), b = int(p / (size_t(Ws) * 2 * H));
+        const float4 v = reinterpret_cast<const float4*>(dx + ((size_t(b) * H + (ys >> 1)) * W + (xs >> 1)) * C)[c];
+        float4 d = reinterpret_cast<const float4*>(dsrc)[k];
+        d.x += 0.25f * v.x;
+        d.y += 0.25f * v.y;
+        d.z += 0.25f * v.z;
+        d.w += 0.25f * v.w;
+        reinterpret_cast<float4*>(dsrc)[k] = d;
+    }
 }
 
-/** Adam step on FP32 master weights, refreshing the BF16 copy. */
-__global__ void adam_k(float* w, bf16* wb, float* g, float* m1, float* m2, size_t n, float lr, float b1, float b2,
-                       float c1, float c2, float eps) {
-    for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
-        float gv = g[k];
-        float a = b1 * m1[k] + (1.f - b1) * gv;
-        float v = b2 * m2[k] + (1.f - b2) * gv * gv;
-        m1[k] = a;
-        m2[k] = v;
-        float wv = w[k] - lr * (a / c1) / (sqrtf(v / c2) + eps);
-        w[k] = wv;
-        if (wb) wb[k] = __float2bfloat16(wv);
-        g[k] = 0.f;
+/** One parameter array of the optimiser: FP32 master values, their BF16 copy
+ * (or null), gradient and moments. */
+struct AdamArray {
+    float* w;
+    bf16* wb;
+    float *g, *m1, *m2;
+    int n;
+};
+struct AdamArgs {
+    AdamArray a[28];
+    float lr, b1, b2, c1, c2, eps;
+};
+/** Adam step on every parameter array (blockIdx.y), refreshing the BF16
+ * copies and clearing the gradients. */
+__global__ void adam_k(const __grid_constant__ AdamArgs p) {
+    const AdamArray& q = p.a[blockIdx.y];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < q.n; k += gridDim.x * blockDim.x) {
+        float gv = q.g[k];
+        float a = p.b1 * q.m1[k] + (1.f - p.b1) * gv;
+        float v = p.b2 * q.m2[k] + (1.f - p.b2) * gv * gv;
+        q.m1[k] = a;
+        q.m2[k] = v;
+        float wv = q.w[k] - p.lr * (a / p.c1) / (sqrtf(v / p.c2) + p.eps);
+        q.w[k] = wv;
+        if (q.wb) q.wb[k] = __float2bfloat16(wv);
+        q.g[k] = 0.f;
     }
 }
 
@@ -755,7 +777,10 @@ __global__ void mse_k(const float* y, const float* t, float* dy, int npx, int C,
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
         float d = y[size_t(p) * C] - t[p];
         s += d * d;
-        dy[size_t(p) * C] = 2.f * d / npx;
+        // the other channels have no target: C (a multiple of 4) values a pixel
+        float4* o = reinterpret_cast<float4*>(dy + size_t(p) * C);
+        o[0] = make_float4(2.f * d / npx, 0.f, 0.f, 0.f);
+        for (int q = 1; q < C / 4; q++) o[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
@@ -770,8 +795,9 @@ __global__ void mse_k(const float* y, const float* t, float* dy, int npx, int C,
 /** Packs a one-channel FP32 image into the 16-channel BF16 network input. */
 __global__ void pack_input_k(const float* x, bf16* in, size_t npx) {
     for (size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < npx; p += size_t(gridDim.x) * blockDim.x) {
-        in[p * 16] = __float2bfloat16(x[p]);
-        for (int c = 1; c < 16; c++) in[p * 16 + c] = __float2bfloat16(0.f);
+        uint4* o = reinterpret_cast<uint4*>(in + p * 16);
+        o[0] = make_uint4(__bfloat16_as_ushort(__float2bfloat16(x[p])), 0, 0, 0);
+        o[1] = make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -983,19 +1009,42 @@ static int net_forward(Net* n, cudaStream_t s, int B, bool keep_fp32_out) {
     return VDI_OK;
 }
 
-/** d += g where the ReLU mask (the layer output) is positive. */
-__global__ void masked_add_k(float* d, const float* g, const bf16* mk, size_t n) {
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-        if (__bfloat162float(mk[i]) > 0.f) d[i] += g[i];
+/** d = g where the ReLU mask (the layer output) is positive, else zero; n a
+ * multiple of 8. */
+__global__ void masked_copy_k(float* __restrict__ d, const float* __restrict__ g, const bf16* __restrict__ mk, size_t n) {
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n / 8; i += size_t(gridDim.x) * blockDim.x) {
+        const uint4 mv = reinterpret_cast<const uint4*>(mk)[i];
+        const bf16* m = reinterpret_cast<const bf16*>(&mv);
+        const float4 a = reinterpret_cast<const float4*>(g)[2 * i], b = reinterpret_cast<const float4*>(g)[2 * i + 1];
+        float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (!(__bfloat162float(m[k]) > 0.f)) f[k] = 0.f;
+        reinterpret_cast<float4*>(d)[2 * i] = make_float4(f[0], f[1], f[2], f[3]);
+        reinterpret_cast<float4*>(d)[2 * i + 1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
 }
 
 /** Backward pass from the gradient in gact[NL-1]; accumulates weight and
- * bias gradients. */
+ * bias gradients. Each output's gradient is written by its first contribution
+ * (the skip's, where there is one, which comes from a later layer; else the
+ * next layer's input gradient), so nothing is cleared first: direct inputs get
+ * their gradient from the convolution itself, upsampled and pooled ones (the
+ * pooled are the outputs with a skip) through one more pass. Adding the pooled
+ * ones in the convolution's epilogue was slower (155 us instead of 37 and the
+ * pass, 64 -> 32 channels at 64 x 128). */
 static int net_backward(Net* n, cudaStream_t s, int B) {
-    for (int k = 0; k < NL - 1; k++) {
+    FlipArgs fa;
+    int most = 0;
+    for (int k = 0; k < NL; k++) {
         const Layer& l = n->L[k];
-        VDI_CUDA(cudaMemsetAsync(n->gact[k], 0, sizeof(float) * size_t(B) * l.H * l.W * l.cout, s));
+        fa.w[k] = l.wb;
+        fa.wt[k] = l.wt;
+        fa.cin[k] = l.cin;
+        fa.cout[k] = l.cout;
+        most = std::max(most, 9 * l.cin * l.cout);
     }
+    flip_transpose_k<<<dim3((most + 255) / 256, NL), 256, 0, s>>>(fa);
     for (int k = NL - 1; k >= 0; k--) {
         const Layer& l = n->L[k];
         const bf16* ymask = l.relu ? n->act[k] : nullptr;
@@ -1003,18 +1052,19 @@ static int net_backward(Net* n, cudaStream_t s, int B) {
         // skip connection: its gradient is the output gradient through the ReLU
         if (l.skip >= 0) {
             size_t na = size_t(B) * l.H * l.W * l.cout;
-            masked_add_k<<<592, 256, 0, s>>>(n->gact[l.skip], dy, ymask, na);
+            masked_copy_k<<<1184, 256, 0, s>>>(n->gact[l.skip], dy, ymask, na);
             VDI_CUDA(cudaGetLastError());
         }
         // weight and bias gradients
         VDI_CUDA(wgrad_dispatch(s, l, layer_input(n, k), dy, ymask, B));
         if (k == 0) continue;   // no gradient needed for the network input
-        // input gradient on the operating grid, then the resampling adjoint
-        int blocks = (9 * l.cin * l.cout + 255) / 256;
-        flip_transpose_k<<<blocks, 256, 0, s>>>(l.wb, l.wt, l.cin, l.cout);
-        ConvArgs<float, float> a{dy, ymask, SRC_DIRECT, l.wt, nullptr, nullptr, 0, n->tmp, B, l.H, l.W};
+        // input gradient on the operating grid, through the resampling's adjoint
+        const bool direct = l.mode == SRC_DIRECT;
+        ConvArgs<float, float> a{dy, ymask, SRC_DIRECT, l.wt, nullptr, nullptr, 0, direct ? n->gact[l.src] : n->tmp,
+                                 B,  l.H,   l.W};
         VDI_CUDA(conv_dispatch(s, l.cout, l.cin, a));
-        resample_adjoint_add_k<<<592, 256, 0, s>>>(n->tmp, n->gact[l.src], l.mode, B, l.H, l.W, l.cin);
+        if (l.mode == SRC_UP2) upsample_adjoint_k<<<1184, 256, 0, s>>>(n->tmp, n->gact[l.src], B, l.H, l.W, l.cin);
+        if (l.mode == SRC_POOL2) pool_adjoint_add_k<<<1184, 256, 0, s>>>(n->tmp, n->gact[l.src], B, l.H, l.W, l.cin);
         VDI_CUDA(cudaGetLastError());
     }
     return VDI_OK;
@@ -1098,19 +1148,26 @@ int vdi_unet_train_step(vdi_unet* u, const float* d_in, const float* d_target, i
     pack_input_k<<<592, 256, 0, s>>>(d_in, n->in, npx);
     VDI_TRY(net_forward(n, s, batch, true));
     VDI_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
-    VDI_CUDA(cudaMemsetAsync(n->gact[NL - 1], 0, sizeof(float) * npx * 16, s));
     mse_k<<<592, 256, 0, s>>>(n->outf, d_target, n->gact[NL - 1], int(npx), 16, n->loss);
     VDI_CUDA(cudaGetLastError());
     VDI_TRY(net_backward(n, s, batch));
     n->step++;
     const float b1 = 0.9f, b2 = 0.999f;
     float c1 = 1.f - std::pow(b1, float(n->step)), c2 = 1.f - std::pow(b2, float(n->step));
+    static_assert(sizeof(AdamArgs::a) / sizeof(AdamArray) == 2 * NL, "weights and biases of every layer");
+    AdamArgs aa;
     for (int k = 0; k < NL; k++) {
-        Layer& l = n->L[k];
-        size_t nw = size_t(9) * l.cin * l.cout;
-        adam_k<<<148, 256, 0, s>>>(l.w, l.wb, l.g, l.m1, l.m2, nw, lr, b1, b2, c1, c2, 1e-8f);
-        adam_k<<<1, 64, 0, s>>>(l.b, nullptr, l.gb, l.bm1, l.bm2, size_t(l.cout), lr, b1, b2, c1, c2, 1e-8f);
+        const Layer& l = n->L[k];
+        aa.a[2 * k] = AdamArray{l.w, l.wb, l.g, l.m1, l.m2, 9 * l.cin * l.cout};
+        aa.a[2 * k + 1] = AdamArray{l.b, nullptr, l.gb, l.bm1, l.bm2, l.cout};
     }
+    aa.lr = lr;
+    aa.b1 = b1;
+    aa.b2 = b2;
+    aa.c1 = c1;
+    aa.c2 = c2;
+    aa.eps = 1e-8f;
+    adam_k<<<dim3(36, 2 * NL), 256, 0, s>>>(aa);
     VDI_CUDA(cudaGetLastError());
     if (loss) {
         VDI_CUDA(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -1135,7 +1192,6 @@ int vdi_unet_gradients(vdi_unet* u, const float* d_in, const float* d_target, in
     pack_input_k<<<592, 256, 0, s>>>(d_in, n->in, npx);
     VDI_TRY(net_forward(n, s, batch, true));
     VDI_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
-    VDI_CUDA(cudaMemsetAsync(n->gact[NL - 1], 0, sizeof(float) * npx * 16, s));
     mse_k<<<592, 256, 0, s>>>(n->outf, d_target, n->gact[NL - 1], int(npx), 16, n->loss);
     VDI_TRY(net_backward(n, s, batch));
     Layer& l = n->L[layer];
