@@ -2578,22 +2578,28 @@ class MG {
         M.off.resize(m);
         M.di.resize(m);
         M.d0.resize(m);
-        M.dt.resize(m);
+        M.ei.resize(m);
+        M.e0.resize(m);
+        M.et.resize(m);
         const double PI = 3.14159265358979323846;
         for (int k = 0; k < m; k++) {
             if (fem()) {
                 // cos(pi k / (m-1)) of the nodes' x neighbours; half of the
-                // diagonal on the top row
-                const double co = std::cos(PI * k / (m - 1));
+                // excess on the top row. A row's coefficients sum to zero.
+                const double co = std::cos(PI * k / (m - 1)), sn = std::sin(0.5 * PI * k / (m - 1));
                 M.off[k] = fop.fey + 2 * fop.fc * co;
                 M.di[k] = M.d0[k] = fop.fm + 2 * fop.fex * co;
-                M.dt[k] = 0.5 * M.di[k];
+                M.ei[k] = M.off[k] * M.di[k] < 0 ? 4 * std::abs(fop.fex + 2 * fop.fc) * sn * sn
+                                                 : std::abs(M.di[k]) - 2 * std::abs(M.off[k]);
+                M.e0[k] = M.ei[k] + std::abs(M.off[k]);
+                M.et[k] = 0.5 * M.ei[k];
             } else {
                 const double sn = std::sin(0.5 * PI * k / m), lam = -4 * c1 * sn * sn;
                 M.off[k] = c2;
                 M.di[k] = lam - 2 * c2;
                 M.d0[k] = lam - (neumann() ? 1 : 3) * c2;
-                M.dt[k] = lam - c2;
+                M.ei[k] = M.et[k] = -lam;
+                M.e0[k] = M.ei[k] + (neumann() ? 0 : 2 * c2);
             }
         }
         M.pin0 = neumann();
@@ -3037,7 +3043,8 @@ class MG {
                        cudaGraphConditionalHandle v) {
         const int nb = std::max(1, std::min(nblk(size(0) / 2 + 1), 8 * resident_blocks() / 6));
         for (int color = 0; color < 2; color++) dr_relax_k<<<nb, 256, 0, s>>>(ccc<double>(0), z, b, ctl, color);
-        dr_polish_check_k<<<sblk0(), 256, 0, s>>>(ccc<double>(0), z, b, rd, ctl, use_cond, h, v);
+        const DirectCheck k = dr_check_shape(m, n, z, b);
+        dr_polish_check_k<<<k.blocks, 256, 0, s>>>(ccc<double>(0), z, b, k.rows, k.vec, rd, ctl, use_cond, h, v);
         VDI_CUDA(cudaGetLastError());
         return VDI_OK;
     }
@@ -3056,8 +3063,8 @@ class MG {
         if (rx.on) return enqueue_relax(s, b, z, 0, use_cond, h);
         if (direct) {
             if (fem())
-                return dr_enqueue(s, femc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, nb, use_cond, h);
-            return dr_enqueue(s, ccc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, nb, use_cond, h);
+                return dr_enqueue(s, femc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, use_cond, h);
+            return dr_enqueue(s, ccc<double>(0), dr, dr_blue, direct_decades(), z, b, rd, ctl, use_cond, h);
         }
         if (precision == VDI_MG_MIXED && !general) {
             if (fem()) first_check_k<double><<<nb, 256, 0, s>>>(femc<double>(0), z, b, rd, ctl, use_cond, h, b32[0]);
