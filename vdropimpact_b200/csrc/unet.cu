@@ -226,6 +226,16 @@ __device__ __forceinline__ uint4 src8_at(const bf16* src, int mode, int H, int W
 // share an SM (tc_blocks), so one's staging and epilogue overlap another's
 // MMAs. Each segment is 9 * CIN/16 MMAs (K = 16 each) into one accumulator, read back
 // with tcgen05.ld for the bias, skip-add, ReLU epilogue.
+// A launch on one image is bound by latency (8 to 14 us each at 256 x 512,
+// where the bytes take 1): so the weights and every row that is read as it
+// is, upsampled ones too, come by asynchronous copies through L1 (the CTAs of
+// an SM share the weights; past L1 the 16-channel layers took 14 us in place
+// of 11), the skip's values are fetched while the MMAs run, and a forward
+// call's launches set up while the ones before them run. A forward call of 1
+// image takes 146 us with these, 240 without; a training step of 8 2.42 and
+// 2.57 ms. CTAs of two launches then share an SM: shared memory holds at most
+// four, of 64 tensor-memory columns at most, so that no allocation of columns
+// waits on a launch that waits itself.
 namespace tc {
 
 constexpr int TC_M = 128;            // output pixels per segment (MMA M)
@@ -290,6 +300,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
     }
 }
 
+/** Asynchronous 16-byte copy to shared memory of `bytes` bytes (16, or 0 for
+ * zeros). */
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
 /** 16 consecutive FP32 accumulator columns of this thread's TMEM lane. */
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     uint32_t r[16];
@@ -337,12 +353,18 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
     unsigned char* rows = smem + 9 * WTAPB;                  // ring [TC_RING][KC][TC_PX][8] bf16
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_slot;
+    __shared__ float bias_s[COUT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the next launch may set up beside this one; it waits below for this
+    // one's results
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#pragma unroll 4
     for (int q = tid; q < 9 * COUT * KC; q += TC_THREADS) {
         const int kc = q % KC, co = (q / KC) % COUT, t = q / (KC * COUT);
-        *reinterpret_cast<uint4*>(wsm + (uint32_t(t) * KC + kc) * COUT * 16 + co * 16) =
-            *reinterpret_cast<const uint4*>(a.w + (size_t(t) * COUT + co) * CIN + kc * 8);
+        cp_async16(wsm + (uint32_t(t) * KC + kc) * COUT * 16 + co * 16, a.w + (size_t(t) * COUT + co) * CIN + kc * 8,
+                   16);
     }
+    if (tid < COUT) bias_s[tid] = a.bias ? a.bias[tid] : 0.f;
     const uint32_t bar_a = smem_u32(&bar);
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
@@ -370,19 +392,18 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
         unsigned char* dst = rows + uint32_t((yy + 1 + TC_RING) % TC_RING) * ROWB;
         const bool rin = yy >= 0 && yy < a.H;
         if constexpr (std::is_same<TIN, bf16>::value) {
-            if (a.mode == SRC_DIRECT) {
-                const bf16* row = a.src + (size_t(b) * a.H + (rin ? yy : 0)) * a.W * CIN;
+            if (a.mode != SRC_POOL2) {
+                const int up = a.mode == SRC_UP2;   // a pixel of the source covers 2 x 2
+                const bf16* row = a.src + (size_t(b) * (a.H >> up) + (rin ? yy >> up : 0)) * (a.W >> up) * CIN;
                 for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
                     const int kc = q % KC, px = q / KC, xx = x0 + px - 1;
                     const bool in = rin && xx >= 0 && xx < a.W;
-                    const int bytes = in ? 16 : 0;   // 0: zero-filled
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                                     smem_u32(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16)),
-                                 "l"(row + (in ? size_t(xx) * CIN + kc * 8 : 0)), "r"(bytes)
-                                 : "memory");
+                    // zero-filled outside the image
+                    cp_async16(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16,
+                               row + (in ? size_t(xx >> up) * CIN + kc * 8 : 0), in ? 16 : 0);
                 }
             } else {
-#pragma unroll 2
+#pragma unroll 3
                 for (int q = tid; q < KC * TC_PX; q += TC_THREADS) {
                     const int kc = q % KC, px = q / KC;
                     *reinterpret_cast<uint4*>(dst + uint32_t(kc) * CHUNKB + uint32_t(px) * 16) =
@@ -418,6 +439,7 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
     };
     uint32_t phase = 0;
     int ok = 1;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the launches before this one, complete
     int pseg = -1, pb = -1, py = -2;   // the previous task, whose next row is staged
     for (long task = t0; task < t1 && ok; task++) {
         const int y = int(task % a.H);
@@ -455,12 +477,18 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
         pseg = seg;
         pb = b;
         py = y;
+        const int x = x0 + warp * 32 + lane;
+        uint4 skip[COUT / 8];
+        if (a.resid && warp < 4 && x < a.W) {
+            const uint4* q = reinterpret_cast<const uint4*>(a.resid + ((size_t(b) * a.H + y) * a.W + x) * COUT);
+#pragma unroll
+            for (int h = 0; h < COUT / 8; h++) skip[h] = q[h];
+        }
         ok = mbar_wait(bar_a, phase) ? 1 : 0;
         phase ^= 1;
         ok = __syncthreads_and(ok);
         fence_after();
         if (ok && warp < 4) {
-            const int x = x0 + warp * 32 + lane;
             const uint32_t ta = tmem + (uint32_t(warp * 32) << 16);
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 16) {
@@ -471,12 +499,12 @@ __global__ void __launch_bounds__(TC_THREADS) conv3x3_tc(ConvArgs<TIN, TOUT> a) 
                     const size_t k = ((size_t(b) * a.H + y) * a.W + x) * COUT + c0;
                     if (a.bias) {
 #pragma unroll
-                        for (int c = 0; c < 16; c++) v[c] += __ldg(a.bias + c0 + c);
+                        for (int c = 0; c < 16; c++) v[c] += bias_s[c0 + c];
                     }
                     if (a.resid) {
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
-                            const uint4 rv = *reinterpret_cast<const uint4*>(a.resid + k + 8 * h);
+                            const uint4 rv = skip[c0 / 8 + h];
                             const bf16* r = reinterpret_cast<const bf16*>(&rv);
 #pragma unroll
                             for (int c = 0; c < 8; c++) v[8 * h + c] += __bfloat162float(r[c]);
@@ -794,6 +822,7 @@ __global__ void mse_k(const float* y, const float* t, float* dy, int npx, int C,
 
 /** Packs a one-channel FP32 image into the 16-channel BF16 network input. */
 __global__ void pack_input_k(const float* x, bf16* in, size_t npx) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < npx; p += size_t(gridDim.x) * blockDim.x) {
         uint4* o = reinterpret_cast<uint4*>(in + p * 16);
         o[0] = make_uint4(__bfloat16_as_ushort(__float2bfloat16(x[p])), 0, 0, 0);
@@ -802,6 +831,7 @@ __global__ void pack_input_k(const float* x, bf16* in, size_t npx) {
 }
 
 __global__ void unpack_output_k(const float* y, float* out, size_t npx) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < npx; p += size_t(gridDim.x) * blockDim.x)
         out[p] = y[p * 16];
 }
@@ -844,8 +874,29 @@ static bool use_tc() {
     return v == 1;
 }
 
+/** Launches a kernel; with early, it may start before the launch ahead of it
+ * in the stream has ended (programmatic dependent launch) and waits itself for
+ * that one's results. What it reads before waiting, the weights, has to be
+ * complete before the launch ahead starts: that one was launched in the plain
+ * way, or behind a plain launch that is behind the weights' last writer. */
+template <class... P, class... A>
+static cudaError_t launch_early(cudaStream_t s, bool early, void (*kernel)(P...), int grid, int threads, size_t smem,
+                                const A&... a) {
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.gridDim = dim3(unsigned(grid));
+    c.blockDim = dim3(unsigned(threads));
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(a)...);
+}
+
 template <int CIN, int COUT, typename TIN, typename TOUT>
-static cudaError_t conv_launch(cudaStream_t s, const ConvArgs<TIN, TOUT>& a) {
+static cudaError_t conv_launch(cudaStream_t s, const ConvArgs<TIN, TOUT>& a, bool early) {
     if (use_tc()) {
         // one wave of resident CTAs: each takes a contiguous run of tasks and
         // stages the next rows while its MMAs run
@@ -863,8 +914,8 @@ static cudaError_t conv_launch(cudaStream_t s, const ConvArgs<TIN, TOUT>& a) {
         }
         const long tasks = long(a.B) * a.H * ((a.W + tc::TC_M - 1) / tc::TC_M);
         const int grid = int(tasks < resident ? tasks : resident);
-        tc::conv3x3_tc<CIN, COUT, TIN, TOUT><<<grid, tc::TC_THREADS, tc::tc_smem<CIN, COUT>(), s>>>(a);
-        return cudaGetLastError();
+        return launch_early(s, early, tc::conv3x3_tc<CIN, COUT, TIN, TOUT>, grid, tc::TC_THREADS,
+                            tc::tc_smem<CIN, COUT>(), a);
     }
     static bool attr = false;
     if (!attr) {
@@ -879,9 +930,9 @@ static cudaError_t conv_launch(cudaStream_t s, const ConvArgs<TIN, TOUT>& a) {
 }
 
 template <typename TIN, typename TOUT>
-static cudaError_t conv_dispatch(cudaStream_t s, int cin, int cout, const ConvArgs<TIN, TOUT>& a) {
+static cudaError_t conv_dispatch(cudaStream_t s, int cin, int cout, const ConvArgs<TIN, TOUT>& a, bool early) {
 #define VDI_CONV(CI, CO) \
-    if (cin == CI && cout == CO) return conv_launch<CI, CO, TIN, TOUT>(s, a);
+    if (cin == CI && cout == CO) return conv_launch<CI, CO, TIN, TOUT>(s, a, early);
     VDI_CONV(16, 16) VDI_CONV(16, 32) VDI_CONV(32, 32) VDI_CONV(32, 64) VDI_CONV(64, 64) VDI_CONV(64, 32)
     VDI_CONV(32, 16)
 #undef VDI_CONV
@@ -993,19 +1044,30 @@ static int net_create(int H, int W, int Bmax, unsigned seed, Net** out) {
 
 static const bf16* layer_input(const Net* n, int k) { return n->L[k].src < 0 ? n->in : n->act[n->L[k].src]; }
 
-static int net_forward(Net* n, cudaStream_t s, int B, bool keep_fp32_out) {
+/** The network on an FP32 image batch, its input packed and (with out) its
+ * output unpacked. Each launch behind the first starts beside the one before
+ * it (16 launches of 2-3 us of set-up each),
+ * but in a stream that is being captured: there the edges stay plain, as a
+ * conditional node's body needs them. */
+static int net_forward(Net* n, cudaStream_t s, const float* in, float* out, int B) {
+    cudaStreamCaptureStatus cap;
+    VDI_CUDA(cudaStreamIsCapturing(s, &cap));
+    const bool early = use_tc() && cap == cudaStreamCaptureStatusNone;
+    const size_t npx = size_t(B) * n->H * n->W;
+    pack_input_k<<<592, 256, 0, s>>>(in, n->in, npx);
+    VDI_CUDA(cudaGetLastError());
     for (int k = 0; k < NL; k++) {
         const Layer& l = n->L[k];
         if (k == NL - 1) {
             ConvArgs<bf16, float> a{layer_input(n, k), nullptr, l.mode, l.wb, l.b, nullptr, 0, n->outf, B, l.H, l.W};
-            VDI_CUDA(conv_dispatch(s, l.cin, l.cout, a));
+            VDI_CUDA(conv_dispatch(s, l.cin, l.cout, a, early));
         } else {
             ConvArgs<bf16, bf16> a{layer_input(n, k), nullptr, l.mode, l.wb, l.b,
                                    l.skip >= 0 ? n->act[l.skip] : nullptr, l.relu, n->act[k], B, l.H, l.W};
-            VDI_CUDA(conv_dispatch(s, l.cin, l.cout, a));
+            VDI_CUDA(conv_dispatch(s, l.cin, l.cout, a, early));
         }
     }
-    (void)keep_fp32_out;
+    if (out) VDI_CUDA(launch_early(s, early, unpack_output_k, 592, 256, 0, n->outf, out, npx));
     return VDI_OK;
 }
 
@@ -1062,7 +1124,7 @@ static int net_backward(Net* n, cudaStream_t s, int B) {
         const bool direct = l.mode == SRC_DIRECT;
         ConvArgs<float, float> a{dy, ymask, SRC_DIRECT, l.wt, nullptr, nullptr, 0, direct ? n->gact[l.src] : n->tmp,
                                  B,  l.H,   l.W};
-        VDI_CUDA(conv_dispatch(s, l.cout, l.cin, a));
+        VDI_CUDA(conv_dispatch(s, l.cout, l.cin, a, false));
         if (l.mode == SRC_UP2) upsample_adjoint_k<<<1184, 256, 0, s>>>(n->tmp, n->gact[l.src], B, l.H, l.W, l.cin);
         if (l.mode == SRC_POOL2) pool_adjoint_add_k<<<1184, 256, 0, s>>>(n->tmp, n->gact[l.src], B, l.H, l.W, l.cin);
         VDI_CUDA(cudaGetLastError());
@@ -1132,11 +1194,7 @@ int vdi_unet_tensor_path(void) { return use_tc() ? 1 : 0; }
 int vdi_unet_forward(vdi_unet* u, const float* d_in, float* d_out, int batch) {
     if (!u || !d_in || !d_out || batch < 1 || batch > u->net->Bmax) return VDI_ERR_INVALID_ARGUMENT;
     Net* n = u->net;
-    size_t npx = size_t(batch) * n->H * n->W;
-    pack_input_k<<<592, 256, 0, u->s>>>(d_in, n->in, npx);
-    VDI_TRY(net_forward(n, u->s, batch, true));
-    unpack_output_k<<<592, 256, 0, u->s>>>(n->outf, d_out, npx);
-    VDI_CUDA(cudaGetLastError());
+    VDI_TRY(net_forward(n, u->s, d_in, d_out, batch));
     return tc_status(u->s);
 }
 
@@ -1145,8 +1203,7 @@ int vdi_unet_train_step(vdi_unet* u, const float* d_in, const float* d_target, i
     Net* n = u->net;
     cudaStream_t s = u->s;
     size_t npx = size_t(batch) * n->H * n->W;
-    pack_input_k<<<592, 256, 0, s>>>(d_in, n->in, npx);
-    VDI_TRY(net_forward(n, s, batch, true));
+    VDI_TRY(net_forward(n, s, d_in, nullptr, batch));
     VDI_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
     mse_k<<<592, 256, 0, s>>>(n->outf, d_target, n->gact[NL - 1], int(npx), 16, n->loss);
     VDI_CUDA(cudaGetLastError());
@@ -1189,8 +1246,7 @@ int vdi_unet_gradients(vdi_unet* u, const float* d_in, const float* d_target, in
         VDI_CUDA(cudaMemsetAsync(l.g, 0, sizeof(float) * 9 * l.cin * l.cout, s));
         VDI_CUDA(cudaMemsetAsync(l.gb, 0, sizeof(float) * l.cout, s));
     }
-    pack_input_k<<<592, 256, 0, s>>>(d_in, n->in, npx);
-    VDI_TRY(net_forward(n, s, batch, true));
+    VDI_TRY(net_forward(n, s, d_in, nullptr, batch));
     VDI_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), s));
     mse_k<<<592, 256, 0, s>>>(n->outf, d_target, n->gact[NL - 1], int(npx), 16, n->loss);
     VDI_TRY(net_backward(n, s, batch));
@@ -1278,10 +1334,7 @@ int unet_correct(vdi_unet* u, cudaStream_t s, const double* r, const double* d_r
         return VDI_ERR_INVALID_ARGUMENT;
     }
     restrict_residual_k<<<592, 256, 0, s>>>(r, d_rnorm, in_buf, m, n, factor);
-    size_t npx = size_t(net->H) * net->W;
-    pack_input_k<<<592, 256, 0, s>>>(in_buf, net->in, npx);
-    VDI_TRY(net_forward(net, s, 1, true));
-    unpack_output_k<<<592, 256, 0, s>>>(net->outf, out_buf, npx);
+    VDI_TRY(net_forward(net, s, in_buf, out_buf, 1));
     prolong_correction_k<<<1184, 256, 0, s>>>(out_buf, d_rnorm, z, m, n, factor, scale);
     VDI_CUDA(cudaGetLastError());
     return VDI_OK;
