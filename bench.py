@@ -6,16 +6,16 @@ One step = fluid_2d::step_forward: gas-layer Newton/tridiagonal update,
 Godunov advection, MAC multigrid projection, two implicit viscous multigrid
 solves, FEM multigrid projection. Solver configurations timed on the same
 workload:
-  plain     - FP64 V-cycles, linear time-extrapolated initial guess (the
-              reference's method on the GPU)
-  fast      - the headline: by default FP32 V-cycles in FP64 iterative
-              refinement with the quadratic time-extrapolated guess, the
-              fastest measured configuration (every solve still stops on the
-              FP64 residual)
-  variants  - the other configurations on the same steps: FP32 coarse-grid
-              corrections (hybrid), FP64 V-cycles (fp64), FP32 V-cycles in
-              FP64 refinement (mixed, when not the headline), and the learned
-              U-Net guess with the refined V-cycles (learned_mixed)
+  plain     - FP64, linear time-extrapolated initial guess (the reference's
+              guess)
+  fast      - the headline: by default the quadratic time-extrapolated guess
+              and mixed precision (every solve stops on the FP64 residual)
+  variants  - the other configurations on the same steps: fp64, hybrid and
+              mixed (when not the headline), and the learned U-Net guess
+              (learned_mixed)
+On this grid every configuration solves the MAC and FEM systems exactly and
+the viscous ones by SOR, both in FP64; the precision names the V-cycles that
+finish what rounding leaves above the tolerance.
 `value` is the headline configuration's steps/s, summed over ranks (each
 rank runs an independent replica of the simulation).
 
@@ -270,38 +270,60 @@ CC_POST_DRAM_BYTES = 192.3e6 / 4
 CC_POST32_DRAM_BYTES = 18.92e6
 
 
+# Algorithmic words (8 bytes) a point: of an exact MAC or FEM solve (b and z
+# read by the transform and by the check, the modal array written, updated and
+# read, z updated) and of one pass of the viscous relaxation (z and b read, z
+# written, for four sweeps).
+EXACT_WORDS = 9
+RELAX_WORDS = 3
+
+
 def roofline(V, torch, args):
-    """The dominant kernel of the step, timed with CUDA events on its own
-    stream over repeated launches at the bench grid: the finest-level
-    post-smoothing tile kernel of the cell-centred solves (MAC and both
-    viscous systems), in the headline's V-cycle precision. Algorithmic
-    bytes per launch: z in, b in, z out plus the coarse correction, 8 bytes
-    a value in FP64 V-cycles, 4 in the FP32 V-cycles of the refinement."""
+    """The kernel with the largest share of the step, the relaxation pass of
+    the viscous systems, timed with CUDA events over whole solves at the bench
+    grid and the workload's coupling: the events also see a solve's launch and
+    the read of its status. Beside it the V-cycles' finest-level
+    post-smoothing tile, which runs where the exact solve or the relaxation
+    does not apply."""
     m, n = (int(x) for x in args.grid.split("x"))
-    s = V.MgsMac(m, n, 1.0 / m, 1.0 / m)
+    peak, kind = measured_peak_gbs()
+    s = V.ViscoImpl(m, n, True, True, 0.4, 0.4)
     g = torch.Generator(device="cuda").manual_seed(0)
     s.b.copy_(torch.randn(m * n, dtype=torch.float64, device="cuda", generator=g))
-    f32 = args.fast_precision == "mixed"
-    ms, nbytes = s.profile(5 if f32 else 1, 100)
-    peak, kind = measured_peak_gbs()
+    e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
+    ms = passes = 0
+    for rep in range(23):
+        s.z.copy_(s.b)
+        flush.zero_()
+        torch.cuda.synchronize()
+        e0.record()
+        v, _ = s.solve_v_cycle(rtol=args.rtol)
+        e1.record()
+        e1.synchronize()
+        if rep >= 3:
+            ms += e0.elapsed_time(e1)
+            passes += v
+    ms /= passes
+    nbytes = RELAX_WORDS * 8 * m * n
     achieved = nbytes / (ms * 1e-3) / 1e9
-    name = "cc_tile<float, POST> (FP32 V-cycle of the refinement)" if f32 else "cc_tile<double, POST>"
-    out = {"kernel": f"{name} on the {args.grid} MAC grid", "bound": "hbm", "achieved": achieved,
-           "peak": peak, "peak_source": kind, "unit": "GB/s", "frac": achieved / peak,
-           "traffic": CC_POST32_DRAM_BYTES if f32 else CC_POST_DRAM_BYTES, "algorithmic_bytes": nbytes,
-           "ms_per_launch": ms}
-    if f32:
-        # the FP64 tile of the FP64 configurations, for comparison
-        ms64, nb64 = s.profile(1, 100)
-        a64 = nb64 / (ms64 * 1e-3) / 1e9
-        out["fp64_tile"] = {"kernel": f"cc_tile<double, POST> on the {args.grid} MAC grid", "achieved": a64,
-                            "frac": a64 / peak, "traffic": CC_POST_DRAM_BYTES, "algorithmic_bytes": nb64,
-                            "ms_per_launch": ms64}
+    out = {"kernel": f"cc_stream_k on the {args.grid} grid (four red-black SOR sweeps a pass)",
+           "bound": "instruction issue and latency", "achieved": achieved, "peak": peak, "peak_source": kind,
+           "unit": "GB/s", "frac": achieved / peak, "algorithmic_bytes": nbytes, "ms_per_launch": ms,
+           "l2": "flushed before each solve"}
+    del s
+    s = V.MgsMac(m, n, 1.0 / m, 1.0 / m)
+    s.b.copy_(torch.randn(m * n, dtype=torch.float64, device="cuda", generator=g))
+    for name, part, traffic in (("float", 5, CC_POST32_DRAM_BYTES), ("double", 1, CC_POST_DRAM_BYTES)):
+        ms, nbytes = s.profile(part, 100)
+        a = nbytes / (ms * 1e-3) / 1e9
+        out[f"vcycle_tile_{name}"] = {"kernel": f"cc_tile<{name}, POST> on the {args.grid} MAC grid", "achieved": a,
+                                      "frac": a / peak, "traffic": traffic, "algorithmic_bytes": nbytes,
+                                      "ms_per_launch": ms}
     return out
 
 
-# Canonical algorithmic bytes of the step's work outside the multigrid
-# V-cycles, per liquid cell, 8-byte words: advection to the MAC source 10,
+# Algorithmic bytes of the step's work outside the solves, per liquid cell, 8-byte words: advection to the MAC source 10,
 # MAC correction and advective update 11, two viscous sources 4, FEM source
 # 3, velocity/pressure update 6 (34 words); and per point of each solve the
 # time-extrapolated initial guess (4 words).
@@ -310,20 +332,21 @@ GUESS_WORDS_PER_POINT = 4
 
 
 def canonical_step(f, res, peak):
-    """Step-level roofline with canonical bytes: the non-multigrid work, the
-    guesses, and every V-cycle taken in the timed window at its hierarchy's
-    canonical bytes per iteration."""
+    """Step-level roofline with algorithmic bytes: the work outside the
+    solves, the guesses, an exact solve a MAC or FEM system and the counted
+    passes of the viscous ones. (The count of an exact solve, the V-cycles it
+    stands for, is not work that was done.)"""
     st = res["stats"]
     steps = max(st["steps"], 1)
-    per_iter = res["vcycle_bytes"]
     cells = f.m * f.n
     pts = {"MAC": cells, "FEM": (f.m + 1) * (f.n + 1), "VX": cells, "VY": cells}
-    mg = sum(st["vcycles"][k] * per_iter[k] for k in per_iter) / steps
+    mg = sum(st["solves"][k] * pts[k] for k in ("MAC", "FEM")) * EXACT_WORDS * 8 / steps
+    mg += sum(st["vcycles"][k] * pts[k] for k in ("VX", "VY")) * RELAX_WORDS * 8 / steps
     guess = sum(st["solves"][k] * pts[k] for k in pts) * GUESS_WORDS_PER_POINT * 8 / steps
     other = STEP_WORDS_PER_CELL * 8 * cells
     total = mg + guess + other
     achieved = total / (res["ms"] / res["steps"] * 1e-3) / 1e9
-    return {"bytes_per_step": total, "multigrid_bytes_per_step": mg, "achieved": achieved, "unit": "GB/s",
+    return {"bytes_per_step": total, "solver_bytes_per_step": mg, "achieved": achieved, "unit": "GB/s",
             "frac": achieved / peak}
 
 
@@ -347,10 +370,11 @@ def vcycle_rooflines(V, torch, args, sim, peak):
 def single_projection(V, torch, args, stream, peak):
     """The single-projection workload: the MAC system on a 2048x1024 grid of
     square cells (mgs_mac's operator), source the seeded zero-mean sum of 64
-    Gaussians, solved from zero to 1e-10 in each precision. Reports V-cycles,
-    CUDA-event time per solve and per V-cycle, canonical GB/s, and the
-    max-relative difference from an FP64 solve run on past its tolerance
-    (8 more V-cycles, where the iterates stop changing)."""
+    Gaussians, solved from zero to 1e-10 in each precision. Reports the count
+    (of an exact solve, the V-cycles it stands for), CUDA-event time per solve,
+    the exact solve's algorithmic GB/s, and the max-relative difference from a
+    solve run on past its tolerance (8 V-cycles more, where the iterates stop
+    changing)."""
     m, n = 2048, 1024
     dx = 1. / m
     b = torch.from_numpy(V.projection_source(m, n, seed=2048)).cuda()
@@ -361,7 +385,7 @@ def single_projection(V, torch, args, stream, peak):
     for _ in range(8):
         s.v_cycle()
     zt = s.z.clone()
-    ms64, by64 = s.profile(2, 20)
+    ms64, _ = s.profile(2, 20)
     out = {"grid": f"{m}x{n}", "source": "zero-mean sum of 64 Gaussians, seed 2048", "rtol": 1e-10,
            "ms_per_fp64_vcycle_mg_test": ms64}
     cells = m * n
@@ -376,19 +400,10 @@ def single_projection(V, torch, args, stream, peak):
             e1.record(stream)
             e1.synchronize()
         ms = e0.elapsed_time(e1)
-        pts = by64 / (8 * (3. * 4 + 4.5))
-        if prec == "fp64":
-            per = by64
-        elif prec == "hybrid":
-            per = by64 / 2 + cells * (3. * 4 + 4.5) * 4
-        else:
-            per = by64 / 2 + 40. * cells
         err = float((s.z - zt).abs().max() / zt.abs().max())
-        achieved = v * per / (ms * 1e-3) / 1e9
-        out[prec] = {"vcycles": v, "rel_res": rel, "ms_per_solve": ms, "ms_per_vcycle": ms / v,
-                     "canonical_bytes_per_vcycle": per, "achieved_gbs": achieved, "frac": achieved / peak,
-                     "max_rel_diff_vs_fp64_converged": err}
-    out["levels_points"] = pts
+        achieved = EXACT_WORDS * 8 * cells / (ms * 1e-3) / 1e9
+        out[prec] = {"counted_vcycles": v, "rel_res": rel, "ms_per_solve": ms, "achieved_gbs": achieved,
+                     "frac": achieved / peak, "max_rel_diff_vs_fp64_converged": err}
     return out
 
 
@@ -463,8 +478,7 @@ def main():
         clocks = ClockSampler(local) if name == "fast" or args.only else None
         f, dt, ms, vc, st, ck, solves = time_config(V, torch, text, args, prec, guess, stream, ws, clocks)
         results[name] = dict(ms=ms, vc=vc, clocks=ck, solves=solves, newton=st["newton_steps"],
-                             launches=st["kernel_launches"], stats=st, steps=args.steps,
-                             vcycle_bytes=f.vcycle_bytes())
+                             launches=st["kernel_launches"], stats=st, steps=args.steps)
         if name == modes[-1][0]:
             keep = (f, dt)
         else:
@@ -477,12 +491,14 @@ def main():
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64" if args.fast_precision == "fp64" else "f64+f32", "data": "synthetic",
         "config": {"workload": WORKLOAD, "grid": args.grid, "mg_rtol": args.rtol,
-                   "solver": f"{args.fast_precision} V-cycles, {args.fast_guess} time-extrapolated guess, "
+                   "solver": "exact MAC and FEM solves, SOR viscous solves, behind them "
+                             f"{args.fast_precision} V-cycles, {args.fast_guess} time-extrapolated guess, "
                              "CUDA-graph step" + ("" if args.no_tune else ", autotuned launch shapes"),
                    "l2": "per-step working set (~0.9 GB) exceeds the 126 MB L2",
                    "parallelism": f"replicas x{ws}"},
         "clocks": head["clocks"],
         "vcycles_per_solve": head["vc"],
+        "vcycles_per_solve_note": "exact solves count the V-cycles they stand for, viscous solves their passes",
         "gpu_launches": head["launches"],
     }
     if "plain" in results:
@@ -492,8 +508,7 @@ def main():
         line["speedup_vs_plain_fp64"] = p["ms"] / head["ms"]
     if not args.no_variants and not args.only and ws == 1:
         # the other solver configurations of the metric, on the same workload:
-        # FP32 coarse-grid corrections, FP32 V-cycles in FP64 refinement, FP64
-        # V-cycles, and the learned guess with the refined V-cycles
+        # the other precisions of the V-cycles, and the learned guess
         vsteps = args.steps
         variants = {}
         others = [("hybrid_quadratic", "hybrid", "quadratic"), ("mixed_quadratic", "mixed", "quadratic"),
@@ -511,7 +526,7 @@ def main():
     line["roofline"] = roofline(V, torch, args)
     peak = line["roofline"]["peak"]
     line["roofline"]["canonical"] = {
-        "note": "SURVEY-style canonical bytes (fusion-independent word counts per point) over CUDA-event time",
+        "note": "algorithmic bytes (word counts per point) over CUDA-event time",
         "step": canonical_step(f, head, peak),
         "vcycle": vcycle_rooflines(V, torch, args, f, peak)}
     if "plain" in results:
