@@ -20,17 +20,21 @@
 // outer RX_HALO columns and 9 rows on either side of a chunk are recomputed
 // by the neighbours.
 //
-// Bound: instruction issue and the latency of the phases' dependent updates
-// (180 instructions a step, 55 of them FP64, 2.3 cycles each at 13 warps an
-// SM), times the redundancy of 64/44 columns and (R + 20)/R rows, against 24
-// bytes a point of memory traffic for four sweeps. A pass at 2048 x 1024
-// takes 48 us from cold caches. Whole solves to 1e-10 at vfx = vfy = 0.4,
-// V-cycles against this: 1024 x 512 223 and 131 us, 2048 x 1024 419 and
-// 187 us.
+// Bound: instructions and the latency they wait for (215 a step, 55 of them
+// FP64; 6.3 cycles between a warp's issues at 14 warps an SM, a third of them
+// on the FP64 results just before, IPC 0.4 a scheduler), times the redundancy
+// of 64/44 columns and (R + 20)/R rows, against 24 bytes a point of memory
+// traffic for four sweeps. A pass at 2048 x 1024 takes 43 us, a solve's first
+// 50 (48 and 57 with the diagonals of the edge rows in registers, which
+// spilled; they are looked up in the operator instead). Whole solves to 1e-10
+// at vfx = vfy = 0.4, V-cycles against this: 1024 x 512 223 and 122 us, 2048 x
+// 1024 419 and 171 us.
 //
 // Slower and not kept: four columns a lane at 168 registers (94 us a pass:
-// too few warps for the same chain), and the rows' loop unrolled over a
-// register ring of 14 rows (75 us, instruction fetch).
+// too few warps for the same chain), the rows' loop unrolled over a
+// register ring of 14 rows (75 us, instruction fetch), and two dependent
+// operations a phase instead of four (178 us a solve: one more instruction
+// costs more than the shorter chain gains).
 
 static constexpr int RX_SWEEPS = 4;
 static constexpr int RX_PH = 2 * RX_SWEEPS;         // colour phases
@@ -92,8 +96,8 @@ __device__ __forceinline__ void rx_copy8(uint32_t dst, const double* src, int by
 
 /** What a lane of rx_walk keeps beside its rows. */
 struct RxLane {
-    double iv[2], dg[2];                   // inverse diagonals and diagonals, interior rows
-    double eb[2], et[2], db[2], dt[2];     // the same on the first and last row
+    double iv[2];                          // inverse diagonals on interior rows (0: a column outside)
+    int xc[2];                             // column classes, for the other rows' and the diagonals
     bool use0, use1;                       // columns this lane finishes
     int na, nb;                            // bytes of its two copies of a row (0: outside, zero-filled)
     const double *pz, *pb;                 // its first column of the next row to copy
@@ -130,13 +134,12 @@ __device__ __forceinline__ void rx_steps(const CCc<double>& c, const RelaxArgs& 
     const int m = c.m, n = c.n;
     auto inv = [&](int r, int k) -> double {
         if (!SLOW) return L.iv[k];
-        const double e = r == 0 ? L.eb[k] : L.et[k];
-        const double w = unsigned(r) < unsigned(n) ? L.iv[k] : 0.;
-        return r == 0 || r == n - 1 ? e : w;
+        const bool on = unsigned(r) < unsigned(n) && L.iv[k] != 0.;
+        return on ? c.invd[L.xc[k]][r == 0 ? 0 : (r == n - 1 ? 2 : 1)] : 0.;
     };
     auto diag = [&](int r, int k) -> double {
-        if (!SLOW) return L.dg[k];
-        return r == 0 ? L.db[k] : (r == n - 1 ? L.dt[k] : L.dg[k]);
+        if (!SLOW) return c.d[L.xc[k]][1];
+        return c.d[L.xc[k]][r == 0 ? 0 : (r == n - 1 ? 2 : 1)];
     };
     const double ox = -c.ox, oy = -c.oy;
     // row t + d sits in group (t + d) / 4 of its ring: three base addresses
@@ -231,11 +234,7 @@ __device__ __forceinline__ void rx_walk(const CCc<double>& c, const RelaxArgs& a
         const bool in = k ? in1 : in0;
         const int x = in ? cls(i0 + k, m) : 0;
         L.iv[k] = in ? c.invd[x][1] : 0.;
-        L.eb[k] = in ? c.invd[x][0] : 0.;
-        L.et[k] = in ? c.invd[x][2] : 0.;
-        L.dg[k] = c.d[x][1];
-        L.db[k] = c.d[x][0];
-        L.dt[k] = c.d[x][2];
+        L.xc[k] = x;
     }
     // x0 + t even at the first step of an iteration (x0 is even): step s then
     // updates column s & 1 of the pair. y0 is a multiple of 4.
