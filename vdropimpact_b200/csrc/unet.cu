@@ -857,7 +857,6 @@ struct Net {
     bf16* act[NL];                     // layer outputs (BF16)
     float* outf = nullptr;             // last layer output (FP32)
     float* gact[NL];                   // gradients of layer outputs
-    float* gin = nullptr;              // gradient of the network input (discarded)
     float* tmp = nullptr;              // input-gradient scratch (largest layer input)
     float* loss = nullptr;
     int step = 0;
@@ -1036,7 +1035,7 @@ static int net_create(int H, int W, int Bmax, unsigned seed, Net** out) {
     }
     size_t npx = size_t(Bmax) * H * W;
     if ((st = balloc(n, &n->in, npx * 16)) || (st = falloc(n, &n->outf, npx * 16)) ||
-        (st = falloc(n, &n->gin, npx * 16)) || (st = falloc(n, &n->tmp, npx * 64)) || (st = falloc(n, &n->loss, 1)))
+        (st = falloc(n, &n->tmp, npx * 64)) || (st = falloc(n, &n->loss, 1)))
         return fail(st);
     *out = n;
     return VDI_OK;
