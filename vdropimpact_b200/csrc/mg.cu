@@ -2139,6 +2139,7 @@ class MG {
     FastArrays<float> fc32;
     bool allow_fast = true;      // false where its arrays would need an allocation
     // the exact solve of the finest level (mg_direct.cuh), when the grid has one
+    bool allow_direct = true;    // false where the owner wants the V-cycles' own iterate (mg_create)
     bool direct = false, dr_blue = false;
     DirectPlan dr;
     void* dr_arena = nullptr;
@@ -2568,7 +2569,7 @@ class MG {
             const char* e = getenv(name);
             return e && (atoi(e) != 0) == on;
         };
-        if (!allow_fast || !(mac_like() || fem()) || is("VDI_MG_DIRECT", false) || is("VDI_MG_FAST_COARSE", false) ||
+        if (!allow_fast || !allow_direct || !(mac_like() || fem()) || is("VDI_MG_DIRECT", false) || is("VDI_MG_FAST_COARSE", false) ||
             is("VDI_MG_GENERAL", true))
             return VDI_OK;
         DirectPlan p;
@@ -3103,13 +3104,14 @@ class MG {
     int* err_word = nullptr;   // see mg_set_error_word
 };
 
-int mg_create(int kind, int m, int n, double c1, double c2, int x_sym, MG** out) {
+int mg_create(int kind, int m, int n, double c1, double c2, int x_sym, MG** out, bool exact) {
     if (!out || m < 2 || n < 2 || kind < 0 || kind > 4) {
         set_error("mg_create: invalid arguments");
         return VDI_ERR_INVALID_ARGUMENT;
     }
     MG* g = new MG();
     g->kind = kind; g->m = m; g->n = n; g->c1 = c1; g->c2 = c2; g->x_sym = x_sym;
+    g->allow_direct = exact;
     if (reg_tile_mode() == 3) ptile_prepare();
     int st = g->build_levels();
     if (st == VDI_OK) st = g->alloc();

@@ -574,7 +574,18 @@ int vdi_sim_create(const vdi_params* prm, void* stream, vdi_sim** out) {
     S->d_gstats = reinterpret_cast<GasStats*>(ebuf + 1);
     // the four linear systems (fluid_2d.cc:19-21)
     if ((st = mg_create(VDI_MG_MAC, m, n, g.xxsp, g.yysp, P.x_sym, &S->mg[SOLVER_MAC])) != VDI_OK) return fail(st);
-    if ((st = mg_create(VDI_MG_FEM, m + 1, n + 1, g.dx, g.dy, P.x_sym, &S->mg[SOLVER_FEM])) != VDI_OK)
+    // The step's FEM system keeps its V-cycles unless its tolerance is 1e-12
+    // or below. Its source holds the gas pressure on the bottom row, which
+    // outweighs the rest of ||b||, so what V-cycles leave beside that row
+    // reaches v through dp/dy. Against an exact solve, v moves at 1e-10 by up
+    // to 1.5e-9 of its norm (512 x 256) and 4.6e-8 at single points (2048 x
+    // 1024), at 1e-12 by 2.8e-11 and 4.4e-10: only there do both give the
+    // fields of one run to 1e-9 and 4e-8. (With the V-cycles, MAC's exact
+    // solve and the viscous SOR move v by at most 2.1e-10 and 2e-8; 520 runs,
+    // 64 x 32 to 2048 x 1024.) A step at 1e-10 pays for it: 1250 us in place
+    // of 728 at 2048 x 1024, mixed precision.
+    const bool fem_exact = S->prm.mg_rtol <= 1e-12;
+    if ((st = mg_create(VDI_MG_FEM, m + 1, n + 1, g.dx, g.dy, P.x_sym, &S->mg[SOLVER_FEM], fem_exact)) != VDI_OK)
         return fail(st);
     if (P.implicit_visc) {
         if ((st = mg_create(VDI_MG_VISC_U, m, n, 1., 1., P.x_sym, &S->mg[SOLVER_VX])) != VDI_OK) return fail(st);

@@ -96,8 +96,9 @@ class MG;
 
 /** Creates a multigrid hierarchy. For MAC c1,c2 = xxsp,yysp (squared inverse
  * spacings); FEM c1,c2 = dx,dy;
- * viscous c1,c2 = vfx,vfy. */
-int mg_create(int kind, int m, int n, double c1, double c2, int x_sym, MG** out);
+ * viscous c1,c2 = vfx,vfy. Without exact, MAC and FEM systems are solved by
+ * V-cycles of the asked precision alone, never by the exact solve. */
+int mg_create(int kind, int m, int n, double c1, double c2, int x_sym, MG** out, bool exact = true);
 void mg_destroy(MG* mg);
 /** Re-derives the viscous coefficients (visco_impl::setup_and_solve
  * re-setup when vfx changes, visco_impl.cc:26-30). */
