@@ -339,15 +339,16 @@ GUESS_WORDS_PER_POINT = 4
 
 def canonical_step(f, res, peak):
     """Step-level roofline with algorithmic bytes: the work outside the
-    solves, the guesses, an exact solve a MAC or FEM system and the counted
-    passes of the viscous ones. (The count of an exact solve, the V-cycles it
+    solves, the guesses, an exact solve a MAC or FEM system and the passes of
+    the viscous ones: two a counted pair, but one of each solve's last, the
+    least that the count allows. (The count of an exact solve, the V-cycles it
     stands for, is not work that was done.)"""
     st = res["stats"]
     steps = max(st["steps"], 1)
     cells = f.m * f.n
     pts = {"MAC": cells, "FEM": (f.m + 1) * (f.n + 1), "VX": cells, "VY": cells}
     mg = sum(st["solves"][k] * pts[k] for k in ("MAC", "FEM")) * EXACT_WORDS * 8 / steps
-    mg += sum(st["vcycles"][k] * pts[k] for k in ("VX", "VY")) * RELAX_WORDS * 8 / steps
+    mg += sum(max(2 * st["vcycles"][k] - st["solves"][k], 0) * pts[k] for k in ("VX", "VY")) * RELAX_WORDS * 8 / steps
     guess = sum(st["solves"][k] * pts[k] for k in pts) * GUESS_WORDS_PER_POINT * 8 / steps
     other = STEP_WORDS_PER_CELL * 8 * cells
     total = mg + guess + other
@@ -504,7 +505,7 @@ def main():
                    "parallelism": f"replicas x{ws}"},
         "clocks": head["clocks"],
         "vcycles_per_solve": head["vc"],
-        "vcycles_per_solve_note": "exact solves count the V-cycles they stand for, viscous solves their passes",
+        "vcycles_per_solve_note": "exact solves count the V-cycles they stand for, viscous solves pairs of passes",
         "gpu_launches": head["launches"],
     }
     if "plain" in results:

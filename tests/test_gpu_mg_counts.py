@@ -1,0 +1,38 @@
+"""What solves report and are capped by where the exact solve (csrc/
+mg_direct.cuh) or the SOR passes (csrc/mg_relax.cuh) stand in for V-cycles."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def V():
+    import vdropimpact_b200 as V
+    return V
+
+
+@pytest.mark.parametrize("m,n", [(256, 128), (1024, 512)])
+@pytest.mark.parametrize("vf", [0.4, 2.0, 3.75, 7.5])
+@pytest.mark.parametrize("rtol", [1e-4, 1e-10])
+def test_a_cap_that_vcycles_meet_is_met(V, monkeypatch, m, n, vf, rtol):
+    """A pair of passes (eight sweeps) gains a factor (omega - 1)^8, 0.02 or
+    less where SOR is used, and a V-cycle 0.1 to 0.01 at the same couplings:
+    with the V-cycles' own count as the cap the passes meet the tolerance."""
+    import torch
+    b = V.projection_source(m, n, 3) + 0.01 * np.random.default_rng(3).standard_normal(m * n)
+
+    def solve(cap):
+        s = V.ViscoImpl(m, n, True, True, vf, vf)
+        s.b.copy_(torch.from_numpy(b))
+        out = []
+        for _ in range(2):          # host-driven, then replayed
+            s.z.copy_(s.b)
+            out.append(s.solve_v_cycle(rtol=rtol, max_vcycles=cap))
+        assert out[0] == out[1] and out[0][1] <= rtol
+        return out[0][0]
+
+    monkeypatch.setenv("VDI_MG_SOR", "0")
+    count = solve(200)
+    monkeypatch.delenv("VDI_MG_SOR")
+    assert 1 <= solve(count) <= count

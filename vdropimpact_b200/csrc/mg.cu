@@ -3314,7 +3314,7 @@ int mg_residual(MG* mg, cudaStream_t s, const double* b, const double* z, double
 }
 
 int mg_kernels_per_iteration(const MG* mg, int precision) {
-    if (mg->rx.on) return 1;   // a pass of sweeps counts as one
+    if (mg->rx.on) return 2;   // a pair of passes
     if (mg->general) return mg->gen.kernels_per_vcycle() + 1;
     if (mg->direct) precision = VDI_MG_FP64;
     if (precision == VDI_MG_HYBRID) {

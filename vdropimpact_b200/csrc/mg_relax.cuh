@@ -337,7 +337,10 @@ __global__ void __launch_bounds__(32 * RX_WARPS, 16 / RX_WARPS) cc_stream_k(CCc<
             if (ctl->done) next = RX_STOP;
         }
         if (next == RX_SWEEP) {
-            solve_decide(ctl, tot[2], 1, a.use_cond, a.h);
+            // a pair of passes counts as one V-cycle, an odd last pass too:
+            // the cap is looked at behind the even ones
+            const bool odd = a.role != 2 && tot[2] > ctl->rtol * ctl->rtol * ctl->bnorm2;
+            solve_decide(ctl, tot[2], !odd, a.use_cond, a.h);
             // an odd pass's result moves to the caller's array either way
             if (ctl->done) next = a.role == 2 ? RX_STOP : RX_COPY;
         }
