@@ -36,3 +36,28 @@ def test_a_cap_that_vcycles_meet_is_met(V, monkeypatch, m, n, vf, rtol):
     count = solve(200)
     monkeypatch.delenv("VDI_MG_SOR")
     assert 1 <= solve(count) <= count
+
+
+def test_launches_of_solves_that_end_at_the_first_check(V):
+    """A tolerance of 1 ends every solve of a first step at its first check,
+    but a viscous solve's pair of passes is launched all the same. Against a
+    step whose solves run (the exact solve's four kernels in place of the FEM
+    check, two launches a counted pair) everything else is equal."""
+    import os
+    cfg = open(os.path.join(os.path.dirname(__file__), "golden", "ld_vis100.cfg")).read()
+    cfg = "\n".join([q for q in cfg.splitlines() if not q.startswith("grid_points")] + ["grid_points 64 32"]) + "\n"
+
+    def step(rtol):
+        f = V.Fluid2D(cfg, mg_rtol=rtol)
+        f.init_fields()
+        f.stats(reset=True)
+        f.step_forward(f.frame_dt(), 1)
+        st = f.stats()
+        f.close()
+        return st
+
+    idle, busy = step(1.0), step(1e-12)
+    assert set(idle["vcycles"].values()) == {0} and set(idle["solves"].values()) == {1}
+    pairs = [busy["vcycles"][k] for k in ("VX", "VY")]
+    assert min(pairs) >= 1
+    assert busy["kernel_launches"] - idle["kernel_launches"] == (4 - 1) + sum(2 * (q - 1) for q in pairs)

@@ -657,7 +657,6 @@ __global__ void __launch_bounds__(256, 3) dr_check_k(OP c, const double* __restr
     double total;
     if (grid_sum(s, rd, &total) && threadIdx.x == 0) {
         ctl->it += ctl->direct;
-        ctl->direct_solves += 1;
         ctl->direct_cycles += ctl->direct;
         ctl->direct = 0;
         solve_decide(ctl, total, 0, use_cond, h);
@@ -682,6 +681,8 @@ __global__ void __launch_bounds__(256) dr_relax_k(CCc<double> c, double* __restr
     }
 }
 
+static constexpr int DR_POLISH_LAUNCHES = 3;   // the sweep's two colours and its check
+
 /** The residual norm after that sweep, and the decision; v is the condition
  * of the V-cycle that follows in a captured loop. Without a sweep the V-cycle
  * follows at once. */
@@ -690,7 +691,10 @@ __global__ void __launch_bounds__(256, 3) dr_polish_check_k(CCc<double> c, const
                                                          SolveCtl* ctl, int use_cond, cudaGraphConditionalHandle h,
                                                          cudaGraphConditionalHandle v) {
     if (!ctl->polish) {
-        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(v, 1);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            ctl->more_launches += DR_POLISH_LAUNCHES;
+            if (use_cond) cudaGraphSetConditional(v, 1);
+        }
         return;
     }
     double s = dr_resid_sum(c, z, b, rows, vec);
@@ -698,6 +702,7 @@ __global__ void __launch_bounds__(256, 3) dr_polish_check_k(CCc<double> c, const
     double total;
     if (grid_sum(s, rd, &total) && threadIdx.x == 0) {
         ctl->polish = 0;
+        ctl->more_launches += DR_POLISH_LAUNCHES;
         solve_decide(ctl, total, 0, use_cond, h);
         if (use_cond) cudaGraphSetConditional(v, !ctl->done);
     }

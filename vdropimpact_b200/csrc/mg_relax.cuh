@@ -334,7 +334,10 @@ __global__ void __launch_bounds__(32 * RX_WARPS, 16 / RX_WARPS) cc_stream_k(CCc<
             ctl->done = 0;
             ctl->status = 0;
             solve_decide(ctl, tot[0] == 0. ? 0. : tot[1], 0, a.use_cond, a.h);
-            if (ctl->done) next = RX_STOP;
+            if (ctl->done) {
+                next = RX_STOP;
+                ctl->more_launches += 2;   // this pass and its pair's other, which returns
+            }
         }
         if (next == RX_SWEEP) {
             // a pair of passes counts as one V-cycle, an odd last pass too:

@@ -934,7 +934,7 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
     VDI_CUDA(cudaStreamSynchronize(S->s));
     memset(out, 0, sizeof(*out));
     out->steps = S->steps;
-    long direct[4] = {0, 0, 0, 0};
+    long direct[4] = {0, 0, 0, 0}, more = 0;
     for (int k = 0; k < 4; k++) {
         if (!S->mg[k]) continue;
         SolveCtl c;
@@ -943,11 +943,12 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
         out->vcycles[k] = long(c.vcycles);
         out->last_rel_res[k] = c.last_rel;
         direct[k] = long(c.direct_cycles);
+        more += long(c.more_launches);
         if (reset) {
             c.solves = 0;
             c.vcycles = 0;
-            c.direct_solves = 0;
             c.direct_cycles = 0;
+            c.more_launches = 0;
             VDI_CUDA(cudaMemcpy(mg_ctl(S->mg[k]), &c, sizeof(SolveCtl), cudaMemcpyHostToDevice));
         }
     }
@@ -955,14 +956,15 @@ int vdi_sim_stats(vdi_sim* S, vdi_stats* out, int reset) {
     // MAC correction, two boundary kernels, the FEM source, the velocity update
     // and the final boundary kernel (+1 viscous source when implicit); per
     // solve the initial guess and the start check; per solve-loop iteration
-    // the kernels of its V-cycle;
-    // per step the lift-off search when it is on, the tracers and the two
-    // frame kernels when those are on, and with the learned guess the
-    // residual kernel and the network's correction.
+    // the kernels of its V-cycle, or a pair of SOR passes; what else the
+    // solves launched, as they counted it; per step the lift-off search when
+    // it is on, the tracers and the two frame kernels when those are on, and
+    // with the learned guess the residual kernel and the network's
+    // correction.
     long per_step = 11 - (S->fused_advect ? 2 : 0) + (S->prm.implicit_visc ? 1 : 0) + (S->lcfg.mode != VDI_LIFTOFF_OFF ? 1 : 0) +
                     (S->prm.ntrace > 0 ? 1 : 0) + (S->prm.nif_mode != 0 ? 2 : 0) +
                     (S->prm.mg_guess == VDI_GUESS_LEARNED ? 1 + unet_kernels_per_correction() : 0);
-    long launches = S->steps * per_step;
+    long launches = S->steps * per_step + more;
     for (int k = 0; k < 4; k++) {
         if (!S->mg[k]) continue;
         // the guess kernel and the solve's start; the V-cycles an exact

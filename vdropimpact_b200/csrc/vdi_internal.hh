@@ -57,11 +57,14 @@ struct SolveCtl {
     int* err_out;       // when set, a failing solve also ORs its bits here
     int tma_timeout;    // set when a tile kernel's bulk copy did not arrive in time
     // exact solves of the finest level: the V-cycles the current solve's one
-    // counts as (0: it does not run), and the totals since the last reset
+    // counts as (0: it does not run), and their total since the last reset
     int direct;
     int polish;         // 1 between an exact solve that fell short and the sweep after it
-    long long direct_solves;
     long long direct_cycles;
+    // kernels launched beside those of a solve's start and of its counted
+    // V-cycles since the last reset: sweeps behind exact solves with their
+    // checks, pairs of SOR passes that ended at the first check
+    long long more_launches;
 };
 
 /** Deterministic block-then-grid sum: each block writes one partial, the
