@@ -2471,6 +2471,16 @@ class MG {
     const ClusterPlan& cplan(double*) const { return cl64; }
     const ClusterPlan& cplan(float*) const { return cl32; }
 
+    /** Blocks of the finest level's tile launch (the variant with the
+     * smallest tiles), each of which writes a partial sum of the residual. */
+    int tile_blocks() const {
+        const int tx = fem() ? std::min(FEMTile<double>::TX, FEMReg<double>::TX)
+                             : std::min(CCTile<double, 2>::TX, CCReg<double>::TX);
+        const int ty = fem() ? std::min(FEMTile<double>::TY, FEMReg<double>::TY)
+                             : std::min(CCTile<double, 2>::TY, CCReg<double>::TY);
+        return int(((long(lv[0].m) + tx - 1) / tx) * ((long(lv[0].n) + ty - 1) / ty));
+    }
+
     int alloc() {
         if (neumann()) {
             VDI_CUDA(cudaMalloc(&bproj, size(0) * sizeof(double)));
@@ -2509,7 +2519,7 @@ class MG {
                 VDI_CUDA(cudaMalloc(&b32[l], s * 4));
             }
         }
-        VDI_TRY(reduce_alloc(rd, MAX_PARTIALS));
+        VDI_TRY(reduce_alloc(rd, std::max(MAX_PARTIALS, tile_blocks())));
         VDI_CUDA(cudaMalloc(&ctl, sizeof(SolveCtl)));
         VDI_CUDA(cudaMemset(ctl, 0, sizeof(SolveCtl)));
         VDI_TRY(set_ctl_params(0, rtol, max_it));
