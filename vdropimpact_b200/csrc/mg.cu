@@ -2555,6 +2555,8 @@ class MG {
         if ((kind != VDI_MG_VISC_U && kind != VDI_MG_VISC_V) || m < 3 || n < 3 || !(c1 >= 0 && c2 >= 0)) return VDI_OK;
         const double sum = 2 * (c1 + c2), rho = sum / (1 + sum), om = 2 / (1 + std::sqrt(1 - rho * rho));
         if (!(om - 1 <= 0.6)) return VDI_OK;
+        rx.R = rx_rows(m, n);
+        if (rx.R == 0) return VDI_OK;
         VDI_CUDA(rx_prepare());
         // the odd passes write the finest tiled level's scratch iterate
         if (!general && nmulti64 > 0 && t64[0]) {
@@ -2565,7 +2567,6 @@ class MG {
         }
         rx.rho2 = rho * rho;
         rx.om_inf = om;
-        rx.R = rx_rows(m, n);
         rx.on = true;
         return VDI_OK;
     }

@@ -370,12 +370,16 @@ struct RelaxPlan {
 
 /** Rows of a chunk: about 16 warps an SM, what the registers hold, with at least 8 rows
  * against the 20 steps that a chunk adds, and few enough blocks for the
- * partial sums. */
+ * partial sums; 0 where one chunk a strip is too many (rows of more than
+ * 480,000 points). */
 static int rx_rows(int m, int n) {
-    const long strips = (m + RX_COLS - 1) / RX_COLS;
+    const long strips = (long(m) + RX_COLS - 1) / RX_COLS;
     long R = (strips * n + 2399) / 2400;
     R = (std::min(64L, std::max(8L, R)) + 3) / 4 * 4;   // whole iterations of the walk
-    while (strips * ((n + R - 1) / R) / RX_WARPS + 1 > MAX_PARTIALS / 3) R *= 2;
+    while (strips * ((n + R - 1) / R) / RX_WARPS + 1 > MAX_PARTIALS / 3) {
+        if (R >= n) return 0;
+        R *= 2;
+    }
     return int(R);
 }
 
