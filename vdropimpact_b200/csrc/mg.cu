@@ -2562,7 +2562,13 @@ class MG {
         if (!general && nmulti64 > 0 && t64[0]) {
             rx.tmp = t64[0];
         } else {
-            VDI_CUDA(cudaMalloc(&rx_tmp, size(0) * sizeof(double)));
+            const cudaError_t me = cudaMalloc(&rx_tmp, size(0) * sizeof(double));
+            if (me == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                rx_tmp = nullptr;
+                return VDI_OK;   // no memory for it: V-cycles
+            }
+            VDI_CUDA(me);
             rx.tmp = rx_tmp;
         }
         rx.rho2 = rho * rho;
@@ -2618,6 +2624,7 @@ class MG {
         if (fem()) p.row0 = 2.0 / fop.fm;
         VDI_CUDA(fem() ? dr_prepare<FEMc<double>>(p, blue) : dr_prepare<CCc<double>>(p, blue));
         VDI_TRY(dr_build(p, fem(), blue, M, &dr_arena));
+        if (!dr_arena) return VDI_OK;   // no memory for it: V-cycles
         dr = p;
         dr_blue = blue;
         direct = true;

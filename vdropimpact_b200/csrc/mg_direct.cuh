@@ -860,7 +860,8 @@ static bool dr_sizes(int m, int n, bool node, DirectPlan& p, bool& blue) {
 }
 
 /** Builds the plan's tables on the host and uploads them in one allocation
- * (*arena, freed by the caller); p holds dr_sizes' result. */
+ * (*arena, freed by the caller; null when the device has no room for it); p
+ * holds dr_sizes' result. */
 static int dr_build(DirectPlan& p, bool node, bool blue, const DirectModes& M, void** arena) {
     const int m = p.m, L = p.L, S = p.S;
     const long P = 1L << p.logp, ml = m;
@@ -907,7 +908,12 @@ static int dr_build(DirectPlan& p, bool node, bool blue, const DirectModes& M, v
         std::copy(q.begin(), q.end(), d2(o_bhat));
     }
     unsigned char* dev = nullptr;
-    VDI_CUDA(cudaMalloc(&dev, off + size_t(p.n) * m * 8));
+    const cudaError_t e = cudaMalloc(&dev, off + size_t(p.n) * m * 8);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return VDI_OK;
+    }
+    VDI_CUDA(e);
     *arena = dev;
     VDI_CUDA(cudaMemcpy(dev, host.data(), from_host, cudaMemcpyHostToDevice));
     auto g2 = [&](size_t o) { return reinterpret_cast<const double2*>(dev + o); };
