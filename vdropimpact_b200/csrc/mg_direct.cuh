@@ -49,6 +49,7 @@ struct DirectPlan {
     int L = 0, S = 0;          // rows of a chunk, chunks of a column
     int modes = 0;             // modes a block of dr_modal_k takes
     double row0 = 1;           // factor of the Dirichlet row's source
+    bool pin0 = false;         // mode 0 is singular: solved with its last value zero, then made mean-free
     const double2* tw = nullptr;     // exp(-2 pi i k / P)
     const double2* post = nullptr;   // cells: (cos, sin)(pi k / 2m)
     double norm = 0;                 // 1 / C_k, twice that of the first (nodes: and last) mode
@@ -483,6 +484,24 @@ __global__ void __launch_bounds__(NT, L == 8 ? 2 : (NT == 256 ? 2 : 1)) dr_modal
     for (int i = 0; i < L; i++) {
         if (i < ni) y[i] -= __ldg(P + long(i) * m) * xp + __ldg(Q + long(i) * m) * D;
         else if (i == ni) y[i] = D;
+    }
+    if (p.pin0 && blockIdx.x == 0) {
+        // The pinned solution's mean is arbitrary, as large as z's error was:
+        // added to z it would be rounded at that scale in every later V-cycle.
+        // (m >= 8: the first block's threads all hold a mode.)
+        double t = 0;
+#pragma unroll
+        for (int i = 0; i < L; i++)
+            if (i <= ni) t += y[i];
+        sx[q][1][tid] = t;
+        __syncthreads();
+        if (c == 0) {
+            double mean = 0;
+            for (int r = 0; r < S; r++) mean += sx[q][1][r * C];
+            mean /= p.R;
+#pragma unroll
+            for (int i = 0; i < L; i++) y[i] -= mean;
+        }
     }
 #pragma unroll
     for (int i = 0; i < L; i++)
@@ -921,6 +940,7 @@ static int dr_build(DirectPlan& p, bool node, bool blue, const DirectModes& M, v
     p.tw = g2(o_tw);
     p.post = g2(o_post);
     p.norm = 2.0 / N;
+    p.pin0 = M.pin0;
     p.chirp = g2(o_chirp);
     p.bhat = g2(o_bhat);
     p.off = g1(o_off);
