@@ -333,7 +333,9 @@ int vdi_mg_setup(vdi_mg* mg);
  * finest level is solved exactly in place of V-cycles (MAC and FEM systems of
  * up to a few thousand points a side), vcycles and max_vcycles count that
  * solve as the V-cycles it stands for: one per 1.25 (FEM 2.5) decades of
- * residual. A max_vcycles at or below that count runs V-cycles. Where a
+ * residual. A max_vcycles at or below that count (or too low for the V-cycles
+ * that a residual more than 14 decades too large needs behind it) runs
+ * V-cycles alone. Where a
  * viscous system is relaxed (vfx + vfy up to about 15), two passes of sweeps
  * count as one V-cycle: they gain at least as much, so a max_vcycles that
  * lets the V-cycles meet rtol lets them meet it too. */

@@ -61,3 +61,38 @@ def test_launches_of_solves_that_end_at_the_first_check(V):
     pairs = [busy["vcycles"][k] for k in ("VX", "VY")]
     assert min(pairs) >= 1
     assert busy["kernel_launches"] - idle["kernel_launches"] == (4 - 1) + sum(2 * (q - 1) for q in pairs)
+
+
+@pytest.mark.parametrize("kind,m,n", [("mac", 100, 50), ("mac", 128, 64), ("fem", 101, 51), ("fem", 129, 65),
+                                      ("neumann", 100, 50), ("neumann", 256, 128)])
+@pytest.mark.parametrize("scale", [0.0, 1.0, 1e4, 1e8])
+def test_a_cap_that_vcycles_meet_is_met_by_exact_solves(V, monkeypatch, kind, m, n, scale):
+    """From starts near and far off, with every cap from the V-cycles' own
+    count on: below the exact solve's count (and what has to follow it) the
+    V-cycles run, above it there is room for both. (The far-off Neumann starts
+    that V-cycles alone do not bring to 1e-10 have no such cap.)"""
+    import torch
+    rng = np.random.default_rng(m)
+    b, z0 = rng.standard_normal(m * n), scale * rng.standard_normal(m * n)
+    if kind == "neumann":
+        b -= b.mean()
+        z0 -= z0.mean()
+        if scale == 1e8:
+            pytest.skip("V-cycles stop at the rounding of the mean")
+
+    def solver():
+        s = {"mac": V.MgsMac, "fem": V.MgsFem, "neumann": V.MgsMacNeumann}[kind](m, n, 1. / m, 1. / m)
+        s.b.copy_(torch.from_numpy(b))
+        return s
+
+    def solve(s, cap):
+        s.z.copy_(torch.from_numpy(z0))
+        return s.solve_v_cycle(rtol=1e-10, max_vcycles=cap)
+
+    monkeypatch.setenv("VDI_MG_DIRECT", "0")
+    count = solve(solver(), 200)[0]
+    monkeypatch.delenv("VDI_MG_DIRECT")
+    s = solver()
+    for cap in range(count, count + 40):
+        v, rel = solve(s, cap)
+        assert rel <= 1e-10 and v <= cap, cap

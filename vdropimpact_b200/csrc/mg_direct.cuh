@@ -263,11 +263,16 @@ __device__ void dr_block_sum2(double& a, double& b) {
     }
 }
 
-/** V-cycles that the exact solve stands for in the caller's count and cap:
- * the decades the residual has to fall over those a V-cycle gains. */
+/** V-cycles that the exact solve stands for in the caller's count: the
+ * decades the residual has to fall over those a V-cycle gains. 0 where they,
+ * one V-cycle more, and those for the decades beyond the 14 that rounding
+ * lets the exact solve gain, at 0.8 each, are not all within the cap: V-cycles
+ * alone may then meet a cap that they do not meet behind it. */
 __device__ __forceinline__ int dr_equivalent(const SolveCtl* ctl, double r2, double decades) {
-    const double d = 0.5 * log10(r2 / (ctl->rtol * ctl->rtol * ctl->bnorm2));
-    return max(1, int(ceil(fmin(d, 1e6) / decades)));
+    const double d = fmin(0.5 * log10(r2 / (ctl->rtol * ctl->rtol * ctl->bnorm2)), 1e6);
+    const int e = max(1, int(ceil(d / decades)));
+    const int more = d > 14 ? 1 + int(ceil((d - 14) / 0.8)) : 0;
+    return e + more < ctl->max_it ? e : 0;
 }
 
 /** Blocks of the transform kernels an SM should hold: they are bound by the
@@ -277,7 +282,7 @@ constexpr int dr_min_blocks(int maxt) { return maxt == 256 ? 4 : (maxt == 512 ? 
 /** Residual of rows 2B and 2B + 1 (block B), their norms, and the rows'
  * modal source into p.work. The last block makes the first decision of the
  * solve (a zero source zeroes z) and sets ctl->direct when the exact solve
- * is to run: the count it stands for lies within the V-cycle cap. */
+ * is to run (dr_equivalent). */
 template <int MAXT, class OP, bool BLUE>
 __global__ void __launch_bounds__(MAXT, dr_min_blocks(MAXT)) dr_forward_k(OP c, DirectPlan p, double* __restrict__ z,
                                                     const double* __restrict__ b, Reduce rd, SolveCtl* ctl,
@@ -392,11 +397,7 @@ __global__ void __launch_bounds__(MAXT, dr_min_blocks(MAXT)) dr_forward_k(OP c, 
         ctl->direct = 0;
         ctl->polish = 0;
         solve_decide(ctl, b2 == 0. ? 0. : r2, 0, use_cond, h);
-        if (!ctl->done) {
-            // below the cap, so that a V-cycle may follow
-            const int e = dr_equivalent(ctl, r2, decades);
-            if (e < ctl->max_it) ctl->direct = e;
-        }
+        if (!ctl->done) ctl->direct = dr_equivalent(ctl, r2, decades);
         zero_src = b2 == 0.;
     }
     __syncthreads();
