@@ -27,8 +27,8 @@
 // traffic for four sweeps. A pass at 2048 x 1024 takes 43 us, a solve's first
 // 50 (48 and 57 with the diagonals of the edge rows in registers, which
 // spilled; they are looked up in the operator instead). Whole solves to 1e-10
-// at vfx = vfy = 0.4, V-cycles against this: 1024 x 512 223 and 122 us, 2048 x
-// 1024 419 and 171 us.
+// at vfx = vfy = 0.4, V-cycles against this: 1024 x 512 227 and 121 us, 2048 x
+// 1024 356 and 171 us.
 //
 // Slower and not kept: four columns a lane at 168 registers (94 us a pass:
 // too few warps for the same chain), the rows' loop unrolled over a
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(32 * RX_WARPS, 16 / RX_WARPS) cc_stream_k(CCc<
             solve_decide(ctl, tot[0] == 0. ? 0. : tot[1], 0, a.use_cond, a.h);
             if (ctl->done) {
                 next = RX_STOP;
-                ctl->more_launches += 2;   // this pass and its pair's other, which returns
+                atomicAdd(&ctl->more_launches, 2ull);   // this pass and its pair's other, which returns
             }
         }
         if (next == RX_SWEEP) {

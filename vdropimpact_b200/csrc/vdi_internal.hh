@@ -64,7 +64,7 @@ struct SolveCtl {
     // kernels launched beside those of a solve's start and of its counted
     // V-cycles since the last reset: sweeps behind exact solves with their
     // checks, pairs of SOR passes that ended at the first check
-    long long more_launches;
+    unsigned long long more_launches;
 };
 
 /** Deterministic block-then-grid sum: each block writes one partial, the
