@@ -13,9 +13,9 @@ workload:
   variants  - the other configurations on the same steps: fp64, hybrid and
               mixed (when not the headline), and the learned U-Net guess
               (learned_mixed)
-On this grid every configuration solves the MAC and FEM systems exactly and
-the viscous ones by SOR, both in FP64; the precision names the V-cycles that
-finish what rounding leaves above the tolerance.
+On this grid every configuration solves the MAC system exactly and the viscous
+ones by SOR, both in FP64, and the FEM system by V-cycles of its precision
+(exactly too with --rtol 1e-12 or below).
 `value` is the headline configuration's steps/s, summed over ranks (each
 rank runs an independent replica of the simulation).
 
@@ -54,8 +54,7 @@ def parse():
     ap.add_argument("--only", default="", help="run only 'plain' or 'fast' (profiling)")
     ap.add_argument("--eager", action="store_true", help="launch kernels without CUDA graphs (profiling)")
     ap.add_argument("--fast-precision", default="mixed", choices=["fp64", "mixed", "hybrid"],
-                    help="the headline configuration's V-cycles (mixed: FP32 V-cycles in FP64 refinement, "
-                         "the fastest measured)")
+                    help="the headline configuration's FEM V-cycles (mixed: FP32 V-cycles in FP64 refinement)")
     ap.add_argument("--fast-guess", default="quadratic", choices=["linear", "quadratic", "learned"])
     ap.add_argument("--no-tune", action="store_true",
                     help="keep the default launch shapes instead of the autotuned ones")
@@ -276,7 +275,7 @@ CC_POST_DRAM_BYTES = 192.3e6 / 4
 CC_POST32_DRAM_BYTES = 18.92e6
 
 
-# Algorithmic words (8 bytes) a point: of an exact MAC or FEM solve (b and z
+# Algorithmic words (8 bytes) a point: of an exact solve (b and z
 # read by the transform and by the check, the modal array written, updated and
 # read, z updated) and of one pass of the viscous relaxation (z and b read, z
 # written, for four sweeps).
@@ -309,7 +308,8 @@ def roofline(V, torch, args):
         e1.synchronize()
         if rep >= 3:
             ms += e0.elapsed_time(e1)
-            passes += v
+            # two passes a counted pair, of which the last may end on the first
+            passes += 2 * v - 1
     ms /= passes
     nbytes = RELAX_WORDS * 8 * m * n
     achieved = nbytes / (ms * 1e-3) / 1e9
@@ -339,15 +339,19 @@ GUESS_WORDS_PER_POINT = 4
 
 def canonical_step(f, res, peak):
     """Step-level roofline with algorithmic bytes: the work outside the
-    solves, the guesses, an exact solve a MAC or FEM system and the passes of
-    the viscous ones: two a counted pair, but one of each solve's last, the
-    least that the count allows. (The count of an exact solve, the V-cycles it
-    stands for, is not work that was done.)"""
+    solves, the guesses, an exact solve of the MAC system (its count, the
+    V-cycles it stands for, is not work that was done), the FEM V-cycles, and
+    the passes of the viscous solves: two a counted pair, but one of each
+    solve's last, the least that the count allows."""
     st = res["stats"]
     steps = max(st["steps"], 1)
     cells = f.m * f.n
     pts = {"MAC": cells, "FEM": (f.m + 1) * (f.n + 1), "VX": cells, "VY": cells}
-    mg = sum(st["solves"][k] * pts[k] for k in ("MAC", "FEM")) * EXACT_WORDS * 8 / steps
+    mg = st["solves"]["MAC"] * pts["MAC"] * EXACT_WORDS * 8 / steps
+    if f.prm.mg_rtol > 1e-12:
+        mg += st["vcycles"]["FEM"] * res["vcycle_bytes"]["FEM"] / steps
+    else:
+        mg += st["solves"]["FEM"] * pts["FEM"] * EXACT_WORDS * 8 / steps
     mg += sum(max(2 * st["vcycles"][k] - st["solves"][k], 0) * pts[k] for k in ("VX", "VY")) * RELAX_WORDS * 8 / steps
     guess = sum(st["solves"][k] * pts[k] for k in pts) * GUESS_WORDS_PER_POINT * 8 / steps
     other = STEP_WORDS_PER_CELL * 8 * cells
@@ -485,7 +489,8 @@ def main():
         clocks = ClockSampler(local) if name == "fast" or args.only else None
         f, dt, ms, vc, st, ck, solves = time_config(V, torch, text, args, prec, guess, stream, ws, clocks)
         results[name] = dict(ms=ms, vc=vc, clocks=ck, solves=solves, newton=st["newton_steps"],
-                             launches=st["kernel_launches"], stats=st, steps=args.steps)
+                             launches=st["kernel_launches"], stats=st, steps=args.steps,
+                             vcycle_bytes=f.vcycle_bytes())
         if name == modes[-1][0]:
             keep = (f, dt)
         else:
@@ -496,16 +501,17 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": "steps/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f64" if args.fast_precision == "fp64" else "f64+f32", "data": "synthetic",
+        "vs_baseline": None, "dtype": "f64+f32" if args.fast_precision != "fp64" and args.rtol > 1e-12 else "f64", "data": "synthetic",
         "config": {"workload": WORKLOAD, "grid": args.grid, "mg_rtol": args.rtol,
-                   "solver": "exact MAC and FEM solves, SOR viscous solves, behind them "
-                             f"{args.fast_precision} V-cycles, {args.fast_guess} time-extrapolated guess, "
+                   "solver": "exact MAC solve, SOR viscous solves, "
+                             + (f"{args.fast_precision} FEM V-cycles" if args.rtol > 1e-12 else "exact FEM solve")
+                             + f", {args.fast_guess} time-extrapolated guess, "
                              "CUDA-graph step" + ("" if args.no_tune else ", autotuned launch shapes"),
                    "l2": "per-step working set (~0.9 GB) exceeds the 126 MB L2",
                    "parallelism": f"replicas x{ws}"},
         "clocks": head["clocks"],
         "vcycles_per_solve": head["vc"],
-        "vcycles_per_solve_note": "exact solves count the V-cycles they stand for, viscous solves pairs of passes",
+        "vcycles_per_solve_note": "an exact solve counts the V-cycles it stands for, a viscous solve pairs of passes",
         "gpu_launches": head["launches"],
     }
     if "plain" in results:
@@ -515,7 +521,7 @@ def main():
         line["speedup_vs_plain_fp64"] = p["ms"] / head["ms"]
     if not args.no_variants and not args.only and ws == 1:
         # the other solver configurations of the metric, on the same workload:
-        # the other precisions of the V-cycles, and the learned guess
+        # the other precisions of the FEM V-cycles, and the learned guess
         vsteps = args.steps
         variants = {}
         others = [("hybrid_quadratic", "hybrid", "quadratic"), ("mixed_quadratic", "mixed", "quadratic"),
