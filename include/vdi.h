@@ -68,7 +68,7 @@ typedef struct vdi_params {
     /* numerical options */
     double mg_rtol;           /* relative residual ||b-Az||/||b|| ending a solve (1e-10) */
     int mg_max_vcycles;       /* V-cycle cap per solve (default 200) */
-    int mg_precision;         /* VDI_MG_FP64 or VDI_MG_MIXED */
+    int mg_precision;         /* a vdi_mg_precision */
     int mg_guess;             /* VDI_GUESS_EXTRAPOLATE or VDI_GUESS_LEARNED */
     /* tracers and the non-inertial frame (fileinfo.cc:59, 96-101, 179-191) */
     int ntrace;               /* tracers advected with the flow (0: none) */
@@ -78,6 +78,9 @@ typedef struct vdi_params {
     int nif_a, nif_b;         /* the nif_range window (fileinfo.cc:182-187) */
 } vdi_params;
 
+/* The kind of V-cycles. Systems that are solved exactly or relaxed in place
+ * of V-cycles (see vdi_mg_solve) are solved in FP64 whichever is asked for, as
+ * are the V-cycles behind an exact solve. */
 enum vdi_mg_precision {
     VDI_MG_FP64 = 0,          /* FP64 V-cycles */
     VDI_MG_MIXED = 1,         /* FP32 V-cycles inside FP64 iterative refinement */
@@ -329,16 +332,16 @@ int vdi_mg_destroy(vdi_mg* mg);
 /* tgmg::setup: builds the level hierarchy (also done by create). */
 int vdi_mg_setup(vdi_mg* mg);
 /* tgmg::solve_v_cycle: V-cycles on z (initial guess in, solution out) until
- * ||b-Az||_2 <= rtol*||b||_2; precision is a vdi_mg_precision. Where the
- * finest level is solved exactly in place of V-cycles (MAC and FEM systems of
- * up to a few thousand points a side), vcycles and max_vcycles count that
- * solve as the V-cycles it stands for: one per 1.25 (FEM 2.5) decades of
- * residual. A max_vcycles at or below that count (or too low for the V-cycles
- * that a residual more than 14 decades too large needs behind it) runs
- * V-cycles alone. Where a
- * viscous system is relaxed (vfx + vfy up to about 15), two passes of sweeps
- * count as one V-cycle: they gain at least as much, so a max_vcycles that
- * lets the V-cycles meet rtol lets them meet it too. */
+ * ||b-Az||_2 <= rtol*||b||_2; precision is a vdi_mg_precision.
+ * MAC and FEM systems of up to a few thousand points a side are solved
+ * exactly instead (in a simulation's step the FEM system only where mg_rtol is
+ * 1e-12 or below). vcycles and max_vcycles then count that solve as the
+ * V-cycles it stands for, one per 1.25 (FEM 2.5) decades of residual, and
+ * those that rounding makes run behind it. A max_vcycles that does not leave
+ * room for both runs V-cycles alone.
+ * Viscous systems up to vfx + vfy of about 15 are relaxed instead. Two passes
+ * of four sweeps count as one V-cycle: they gain at least as much, so a
+ * max_vcycles within which V-cycles meet rtol is enough for them. */
 typedef struct vdi_mg_result {
     int vcycles;
     double rel_res;
@@ -425,9 +428,11 @@ int vdi_unet_guess(vdi_unet* net, vdi_mg* mg, int factor, double scale, const do
  * uses one static device array of about 5 MB that every GPU loading the
  * library holds until exit. Grids are limited to 262144 unknowns (m*n);
  * larger ones return VDI_ERR_UNSUPPORTED_SIZE. Its coarsest level is
- * smoothed rather than solved with a precomputed inverse, so its V-cycle
- * count can exceed vdi_mg_solve's (about twice on a 641 x 385 FEM grid,
- * 17 against 9); it stops on the same residual test.
+ * smoothed rather than solved with a precomputed inverse, and MAC and FEM
+ * systems are not solved exactly (viscous ones are relaxed as by
+ * vdi_mg_solve), so its count can exceed vdi_mg_solve's (17 on a 641 x 385
+ * FEM grid, where V-cycles with that inverse take 9 and the exact solve
+ * counts 4); it stops on the same residual test.
  * The first call on a device looks up the array's device address and should
  * come before any stream capture. Calls share the array: two calls that
  * overlapped on the GPU would race on it. The entry point holds a
@@ -440,7 +445,8 @@ int vdi_mg_solve_noalloc(int kind, int m, int n, double c1, double c2, int x_sym
 
 /* ------------------------------------------------------- tridiagonal
  * tri_solve::solve_lapack (tri_solve.cc:24-33): solves the n x n system in
- * place (solution in d_d) on the GPU by cyclic reduction, falling back to
+ * place (solution in d_d) on the GPU: rows eliminated per thread and the rest
+ * reduced in parallel (cyclic reduction beyond 4096 rows), falling back to
  * Gaussian elimination with partial pivoting when a row is not diagonally
  * dominant. a, b, c are overwritten. *pivoted is set to 1 when the fallback
  * ran (may be NULL). */

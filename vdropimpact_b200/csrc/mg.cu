@@ -2543,10 +2543,13 @@ class MG {
     }
 
     /** The SOR solver for the viscous systems (mg_relax.cuh) while its rate,
-     * omega - 1 a sweep, is below 0.6 (vfx + vfy up to 7.5). At 2048 x 1024 a
-     * solve to 1e-10 takes V-cycles 419 us at vfx = vfy = 0.4, 657 at 1 and 829
-     * at 3, this 187 us at 0.4 and 306 at 2; past the line its passes would
-     * outnumber the V-cycles.
+     * omega - 1 a sweep, is at most 0.6 (vfx + vfy up to 15.2). Up to there
+     * two passes gain at least what a V-cycle does, on which their count
+     * rests: 1024 x 512 at vfx = vfy = 7.5 takes 3 pairs or 3 V-cycles to
+     * 1e-4, 6 or 9 to 1e-10; at 15 (past the line) 4 or 3, and 9 or 9. Solves
+     * of 2048 x 1024 to 1e-10, V-cycles and this: 356 and 171 us at vfx = vfy =
+     * 0.4, 677 and 271 at 2, 766 and 353 at 3.75, 971 and 501 at 7.5; past the
+     * line 971 and 697 at 15, 1289 and 1118 at 40.
      * VDI_MG_SOR=0 and VDI_MG_GENERAL turn it off. */
     int setup_relax() {
         const char* e = getenv("VDI_MG_SOR");
@@ -3036,7 +3039,8 @@ class MG {
                      cudaGraphConditionalHandle h) {
         if (rx.on) return enqueue_relax(s, b, z, 2, use_cond, h);
         // what an exact solve leaves is rounding of z, which FP32 corrections
-        // cannot lower: the V-cycles after it are FP64 ones
+        // cannot lower: the V-cycles after it (and those a low cap asks for in
+        // its place) are FP64 ones, whatever precision is asked for
         if (direct) return vcycle64(s, b, z, 1, use_cond, h);
         if (precision == VDI_MG_HYBRID) return vcycle_hybrid(s, b, z, 1, use_cond, h);
         if (precision == VDI_MG_MIXED && !general) {

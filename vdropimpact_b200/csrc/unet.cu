@@ -232,7 +232,7 @@ __device__ __forceinline__ uint4 src8_at(const bf16* src, int mode, int H, int W
 // an SM share the weights; past L1 the 16-channel layers took 14 us in place
 // of 11), the skip's values are fetched while the MMAs run, and a forward
 // call's launches set up while the ones before them run. A forward call of 1
-// image takes 146 us with these, 240 without; a training step of 8 2.42 and
+// image takes 143 us with these, 240 without; a training step of 8 2.42 and
 // 2.57 ms. CTAs of two launches then share an SM: shared memory holds at most
 // four, of 64 tensor-memory columns at most, so that no allocation of columns
 // waits on a launch that waits itself.
